@@ -11,8 +11,8 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(BUILD, "libmdgpu_gb300.so")
 SOURCES = ["md_api.cu", "k_cells.cu", "k_forces.cu", "k_integrate.cu", "k_probe.cu", "k_noalloc.cu", "k_fused.cu",
-           "k_batch.cu", "k_adjoint.cu", "md_compat.cu", "k_pair64.cu", "k_pme.cu"]
-HEADERS = ["md_internal.h", "md_device.cuh", "md_pair.cuh", "md_thermo.cuh",
+           "k_batch.cu", "k_run.cu", "k_adjoint.cu", "md_compat.cu", "k_pair64.cu", "k_pme.cu"]
+HEADERS = ["md_internal.h", "md_device.cuh", "md_pair.cuh", "md_thermo.cuh", "md_rebuild.cuh", "md_bonded.cuh",
            os.path.join("..", "..", "include", "md_gpu.h"), os.path.join("..", "..", "include", "md_gpu_compat.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # cuFFT (the PME transforms) is found there at run time as well

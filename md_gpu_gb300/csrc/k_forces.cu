@@ -16,6 +16,7 @@
  * per-atom lists (each bond seen from both atoms, each angle from all three);
  * the centre-atom branch uses the role of the entry being processed.
  */
+#include "md_bonded.cuh"
 #include "md_pair.cuh"
 
 namespace {
@@ -49,15 +50,8 @@ __global__ void __launch_bounds__(128) k_pair(md_kparams kp, pair_consts pc,
     }
 }
 
-__device__ __forceinline__ void min_image(float &dx, float &dy, float &dz, const float *box, const float *boxi)
-{
-    dx -= box[0] * rintf(dx * boxi[0]);
-    dy -= box[1] * rintf(dy * boxi[1]);
-    dz -= box[2] * rintf(dz * boxi[2]);
-}
-
-/* Harmonic bonds (U = k (r - r0)^2, bnd1 = 2k) and angles (U = k (th - th0)^2,
- * ang1 = 2k), one thread per sorted atom, added into the fixed-point forces.
+/* Bonds and angles (bonded_atom), one thread per sorted atom, added into the
+ * fixed-point forces.
  * In a batch (reps non-null) the minimum image uses the atom's replica box. */
 template <bool ENERGY>
 __global__ void k_bonded(md_kparams kp, const float4 *__restrict__ pos4,
@@ -74,51 +68,8 @@ __global__ void k_bonded(md_kparams kp, const float4 *__restrict__ pos4,
     int na = has_angles ? al_sn[s] : 0;
     if (nb == 0 && na == 0) return;
     const float *box = reps ? reps[arep[s]].box : kp.box, *boxi = reps ? reps[arep[s]].boxi : kp.boxi;
-    const float *bnd1 = par, *bnd2 = par + MD_MAXTYPE, *ang1 = par + 2 * MD_MAXTYPE,
-                *ang2 = par + 3 * MD_MAXTYPE;
-    float4 p = pos4[s];
-    float fx = 0.0f, fy = 0.0f, fz = 0.0f, fw = 0.0f, fe = 0.0f;
-    for (int k = 0; k < nb; k++) {
-        int2 b = bl_s[k * P + s];
-        float4 q = pos4[b.x];
-        float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        min_image(dx, dy, dz, box, boxi);
-        float rsq = dx * dx + dy * dy + dz * dz;
-        float ri = rsqrtf(rsq);
-        float kk = bnd1[b.y], r0 = bnd2[b.y];
-        float fa = kk * (r0 * ri - 1.0f);
-        fw += fa * rsq;
-        fx += fa * dx; fy += fa * dy; fz += fa * dz;
-        if (ENERGY) { float dr = rsq * ri - r0; fe += 0.25f * kk * dr * dr; }
-    }
-    for (int k = 0; k < na; k++) {
-        int4 a = al_s[k * P + s];
-        float4 qa, qb = pos4[a.z];
-        float4 cen;
-        if (a.x == 1) { qa = pos4[a.y]; cen = p; }   /* this atom is the centre */
-        else { qa = p; cen = pos4[a.y]; }           /* this atom is an end */
-        float ax = qa.x - cen.x, ay = qa.y - cen.y, az = qa.z - cen.z;
-        min_image(ax, ay, az, box, boxi);
-        float bx = qb.x - cen.x, by = qb.y - cen.y, bz = qb.z - cen.z;
-        min_image(bx, by, bz, box, boxi);
-        float ai = rsqrtf(ax * ax + ay * ay + az * az);
-        float bi = rsqrtf(bx * bx + by * by + bz * bz);
-        float ab = ax * bx + ay * by + az * bz;
-        float cang = ab * ai * bi;
-        cang = fminf(fmaxf(cang, -0.9999999f), 0.9999999f);
-        float th = acosf(cang);
-        float ff = ang1[a.w] * (th - ang2[a.w]) * rsqrtf(1.0f - cang * cang) * ai * bi;
-        float aa = ab * ai * ai;
-        float gx = bx - aa * ax, gy = by - aa * ay, gz = bz - aa * az;
-        if (a.x == 1) {
-            float bb = ab * bi * bi;
-            gx = bb * bx - ax - gx;
-            gy = bb * by - ay - gy;
-            gz = bb * bz - az - gz;
-        }
-        fx += ff * gx; fy += ff * gy; fz += ff * gz;
-        if (ENERGY) { float dth = th - ang2[a.w]; fe += 0.5f * ang1[a.w] * dth * dth * (1.0f / 3.0f); }
-    }
+    float fx, fy, fz, fw, fe;
+    bonded_atom<ENERGY>(s, P, nb, na, box, boxi, pos4, bl_s, al_s, par, fx, fy, fz, fw, fe);
     f[s] += __float2ll_rn(fx * 4294967296.0f);
     f[P + s] += __float2ll_rn(fy * 4294967296.0f);
     f[2 * P + s] += __float2ll_rn(fz * 4294967296.0f);

@@ -258,7 +258,7 @@ void free_device(md_ctx *c)
                     c->tmp_i, c->bl_o, c->bl_on, c->al_o, c->al_on, c->bl_s, c->bl_sn, c->al_s,
                     c->al_sn, c->st, c->rec, c->lj_dev, c->bonded_par,
                     c->type_mask_dev, c->io_dev, c->reps_dev, c->repst, c->arep, c->crep,
-                    c->ljr_dev, c->grid_tab, c->rep_upd, c->racc, c->p64_dev, c->rep_hist, c->snap};
+                    c->ljr_dev, c->grid_tab, c->rep_upd, c->racc, c->p64_dev, c->rep_hist, c->snap, c->run_ctl};
     for (void *p : ptrs)
         if (p) cudaFree(p);
 }
@@ -569,7 +569,7 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
     MD_ALLOC(c->tmp_d, 8 * P); MD_ALLOC(c->tmp4, P); MD_ALLOC(c->tmp_i, 3 * P);
     MD_ALLOC(c->bl_o, 4 * P); MD_ALLOC(c->bl_on, P); MD_ALLOC(c->al_o, 4 * P); MD_ALLOC(c->al_on, P);
     MD_ALLOC(c->bl_s, 4 * P); MD_ALLOC(c->bl_sn, P); MD_ALLOC(c->al_s, 4 * P); MD_ALLOC(c->al_sn, P);
-    MD_ALLOC(c->st, 1);
+    MD_ALLOC(c->st, 1); MD_ALLOC(c->run_ctl, 128);
     c->rec_cap = 4096;
     MD_ALLOC(c->rec, c->rec_cap);
     MD_ALLOC(c->lj_dev, 2 * MD_MAXTYPE * MD_MAXTYPE);
@@ -608,6 +608,7 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
     auto up = [&](void *dst, const void *srcp, size_t bytes) {
         if (e == cudaSuccess && bytes > 0) e = cudaMemcpy(dst, srcp, bytes, cudaMemcpyHostToDevice);
     };
+    if (e == cudaSuccess) e = cudaMemset(c->run_ctl, 0, 128 * sizeof(unsigned long long));
     up(c->x, h.x.data(), sizeof(double) * 3 * P);
     up(c->v, h.v.data(), sizeof(double) * 3 * P);
     up(c->mass, h.m.data(), sizeof(double) * P);
@@ -1524,11 +1525,37 @@ static md_status sync_reps(md_ctx *c)
     return MD_OK;
 }
 
+/* Steps of a small system from here on that k_run_steps takes in one
+ * launch: up to the next step with energies (which runs as separate
+ * kernels), at most 1024 (a few ms), at least 4. */
+static int run_small_steps(md_ctx *c, int left, int energy_every)
+{
+    int k = std::min(left, 1024);
+    if (energy_every > 0) {
+        const long long past = c->host_step % energy_every;
+        if (past == 0) return 0;
+        k = (int)std::min<long long>(k, energy_every - past);
+    }
+    return k >= 4 && md_can_run_small(c) ? k : 0;
+}
+
 static md_status step_body(md_ctx *c, int nsteps, int energy_every, bool mark_start)
 {
     if (mark_start) MD_CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
     int left = nsteps;
     while (left > 0) {
+        const int small = run_small_steps(c, left, energy_every);
+        if (small > 0 && launch_run_steps(c, md_make_kparams(c), small)) {
+            c->host_step += small;
+            left -= small;
+            continue;
+        }
+        if (energy_every > 4 && c->host_step % energy_every == 0 && md_can_run_small(c)) {
+            enqueue_steps(c, 1, 1);   /* the energy step between two runs of small steps */
+            c->host_step++;
+            left--;
+            continue;
+        }
         int aligned = energy_every > 0 ? (int)(c->host_step % energy_every == 0) : 1;
         int g = energy_every > 0 ? energy_every : std::min(nsteps, 32);
         if (!aligned || left < g || !c->use_graphs) {

@@ -252,6 +252,9 @@ struct md_ctx {
                                       before its first barrier (-1: none) */
     int coop_grid = 0;             /* its blocks (0: not found yet, -1: unavailable) */
     int nsm = 1;                   /* SMs of the device (found with cw_grid) */
+    unsigned long long *run_ctl = nullptr; /* barrier and sums of k_run_steps: two sets of 64 words */
+    int run_parity = 0;            /* the set its next launch uses */
+    int run_key = 0, run_blocks = 0; /* resident blocks of k_run_steps and the lane count they are for */
     int rebuild_inline = 0;        /* step graphs: 1 = list passes inline (programmatic launches
                                       that return at once without a request), 0 = a conditional node */
     long long host_step = 0;       /* steps run so far (mirrors st->step) */
@@ -368,6 +371,10 @@ void launch_scatter_in(md_ctx *c, const md_kparams &kp, int what, const void *sr
 bool md_can_fuse(const md_ctx *c);
 /* Pair forces + leapfrog + check in one kernel; swaps pos4 and pos4_alt. */
 void launch_pair_leapfrog(md_ctx *c, const md_kparams &kp, unsigned long long cond, int has_cond);
+
+/* ---- launchers (k_run.cu): many steps of a small system in one launch ---- */
+bool md_can_run_small(md_ctx *c);
+bool launch_run_steps(md_ctx *c, const md_kparams &kp, int nsteps);
 
 /* ---- launchers of batches (k_batch.cu); the launchers above forward to
  * these for batch contexts (the list kernels of a batch live in k_cells.cu) ---- */

@@ -299,15 +299,22 @@ __device__ __forceinline__ bool interior(const G &g, float4 pi)
            fabsf(pi.z) + rc < 0.499f * g.L(2);
 }
 
+/* A load through the read-only path (NC: data no block writes while the
+ * kernel runs) or an ordinary one (data other blocks wrote before the last
+ * grid barrier of a kernel that runs many steps). */
+template <bool NC, class T>
+__device__ __forceinline__ T ld_list(const T *p)
+{
+    return NC ? __ldg(p) : *p;
+}
+
 /* The entries of one lane in batches of B, software pipelined: while batch
  * t is computed, the positions of batch t+1 and the list entries of batch
  * t+2 are in flight.  ljrow may point into shared memory (a batch's
  * per-replica table): plain loads there, not the read-only global path. */
-template <int KIND, int TPA, int B, bool ENERGY, bool WRAP, bool PACK, int UNROLL, class G>
-__device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int nb,
-                                          const unsigned *__restrict__ lp,
-                                          const float4 *__restrict__ pos4, const float2 *ljrow,
-                                          pair_acc &acc)
+template <int KIND, int TPA, int B, bool ENERGY, bool WRAP, bool PACK, int UNROLL, bool NC, class G>
+__device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int nb, const unsigned *lp,
+                                          const float4 *pos4, const float2 *ljrow, pair_acc &acc)
 {
     unsigned e0[B], e1[B];
     float4 p0[B];
@@ -321,12 +328,12 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
     wrapxy WXY;
     if (!(PACK && !ENERGY && B % 2 == 0) && WRAP) WXY = wrapxy::make(g);
 #pragma unroll
-    for (int b = 0; b < B; b++) e0[b] = __ldg(lp + b * TPA);
+    for (int b = 0; b < B; b++) e0[b] = ld_list<NC>(lp + b * TPA);
 #pragma unroll
-    for (int b = 0; b < B; b++) p0[b] = __ldg(pos4 + (e0[b] & MD_INDEX_MASK));
+    for (int b = 0; b < B; b++) p0[b] = ld_list<NC>(pos4 + (e0[b] & MD_INDEX_MASK));
     if (nb > 1) {
 #pragma unroll
-        for (int b = 0; b < B; b++) e1[b] = __ldg(lp + (B + b) * TPA);
+        for (int b = 0; b < B; b++) e1[b] = ld_list<NC>(lp + (B + b) * TPA);
     }
 #pragma unroll UNROLL
     for (int t = 0; t < nb; t++) {
@@ -334,11 +341,11 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
         unsigned e2[B];
         if (t + 1 < nb) {
 #pragma unroll
-            for (int b = 0; b < B; b++) p1[b] = __ldg(pos4 + (e1[b] & MD_INDEX_MASK));
+            for (int b = 0; b < B; b++) p1[b] = ld_list<NC>(pos4 + (e1[b] & MD_INDEX_MASK));
         }
         if (t + 2 < nb) {
 #pragma unroll
-            for (int b = 0; b < B; b++) e2[b] = __ldg(lp + ((t + 2) * B + b) * TPA);
+            for (int b = 0; b < B; b++) e2[b] = ld_list<NC>(lp + ((t + 2) * B + b) * TPA);
         }
         if (PACK && !ENERGY && B % 2 == 0) {
 #pragma unroll
@@ -381,12 +388,10 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
  * FP32 and converts its sum to int64 once; lane sums are combined with
  * integer shuffles (exact), so the result depends only on TPA.  Every lane of
  * the warp must call this (the shuffles use the full mask). */
-template <int KIND, int TPA, int B, bool ENERGY, bool PACK = true, int UNROLL = 0, class G>
+template <int KIND, int TPA, int B, bool ENERGY, bool PACK = true, int UNROLL = 0, bool NC = true, class G>
 __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool active, int lane,
-                                               const float4 *__restrict__ pos4,
-                                               const int *__restrict__ type,
-                                               const unsigned *__restrict__ nl,
-                                               const int *__restrict__ nl_n, const float2 *lj)
+                                               const float4 *pos4, const int *type, const unsigned *nl,
+                                               const int *nl_n, const float2 *lj)
 {
     static_assert(MD_LIST_QUANTUM % (TPA * B) == 0, "batch must divide the list padding");
     const float4 pi = pos4[ii];
@@ -411,9 +416,9 @@ __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool
     const bool inner = g.centered() && __all_sync(0xffffffffu, !active || interior(g, pi));
     if (nb > 0) {
         if (inner)
-            pair_loop<KIND, TPA, B, ENERGY, false, PACK, UNR>(g, pi, qi, nb, lp, pos4, ljrow, acc);
+            pair_loop<KIND, TPA, B, ENERGY, false, PACK, UNR, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
         else
-            pair_loop<KIND, TPA, B, ENERGY, true, PACK, UNR>(g, pi, qi, nb, lp, pos4, ljrow, acc);
+            pair_loop<KIND, TPA, B, ENERGY, true, PACK, UNR, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
     }
     pair_total r;
     r.fx = __float2ll_rn(acc.fx * 4294967296.0f);

@@ -1,0 +1,70 @@
+"""Many steps of a small system in one launch (k_run_steps): bit for bit the
+run of the separate kernels launched step by step (md_set_graphs off)."""
+import numpy as np
+import pytest
+
+from md_gpu_gb300 import MDSystem, synth
+
+pytestmark = pytest.mark.gpu
+
+# (system, lanes per atom, steps, energy_every): block edges (256 / lanes atoms
+# per block), one atom more and less than a block, the largest system that runs
+# this way, odd and even step counts (position buffers), energy steps between
+CASES = [
+    ("argon", dict(ncell=4), 8, 41, 0),
+    ("argon", dict(ncell=5), 16, 40, 7),
+    ("argon", dict(ncell=9), 32, 33, 16),
+    ("nacl", dict(natom=510), 8, 64, 0),
+    ("nacl", dict(natom=514), 16, 31, 10),
+    ("nacl", dict(natom=9602), 8, 24, 0),
+    ("water", dict(nside=8), 8, 40, 0),
+    ("water", dict(nside=9), 16, 37, 12),
+    ("water", dict(nside=8), 32, 24, 0),
+]
+
+
+def _system(kind, kw, tmp_path):
+    if kind == "argon":
+        return MDSystem.from_arrays(**synth.to_arrays(synth.argon_fcc(seed=3, integrator="vv", **kw)))
+    if kind == "nacl":
+        return MDSystem.from_arrays(**synth.to_arrays(synth.nacl_replica(
+            seed=4, integrator="leapfrog", ensemble="nvt", **kw)))
+    return MDSystem.from_files(synth.write_case(synth.water_grid(seed=5, **kw), str(tmp_path), "w"))
+
+
+@pytest.mark.parametrize("kind,kw,tpa,steps,every", CASES)
+def test_small_run_matches_separate_kernels(kind, kw, tpa, steps, every, tmp_path):
+    out = []
+    for graphs in (True, False):
+        with _system(kind, kw, tmp_path) as sim:
+            sim.set_tuning(tpa, 0)
+            sim.set_graphs(graphs)
+            sim.step(steps, every)
+            mid = [sim.positions(), sim.velocities(), sim.forces()]
+            sim.step(steps, every)
+            out.append(mid + [sim.positions(), sim.velocities(), sim.forces(), sim.order(), sim.history(2 * steps),
+                              sim.info()["builds"]])
+    for k, (a, b) in enumerate(zip(*out)):
+        if isinstance(a, np.ndarray):
+            assert np.array_equal(a, b), f"output {k} differs by {np.abs(a - b).max()}"
+        else:
+            assert a == b
+    assert out[0][-1] >= 2
+
+
+def test_two_small_systems_interleaved():
+    """Runs of two contexts in turn do not see each other's barrier state."""
+    def make(seed):
+        return MDSystem.from_arrays(**synth.to_arrays(synth.argon_fcc(ncell=5, seed=seed, integrator="vv")))
+
+    alone = []
+    for seed in (1, 2):
+        with make(seed) as s:
+            for n in (5, 8, 21):
+                s.step(n)
+            alone.append(s.positions())
+    with make(1) as a, make(2) as b:
+        for n in (5, 8, 21):
+            a.step(n)
+            b.step(n)
+        assert np.array_equal(a.positions(), alone[0]) and np.array_equal(b.positions(), alone[1])
