@@ -194,7 +194,7 @@ __global__ void k_permute(md_kparams kp, const md_devstate *st, int always,
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= kp.n) return;
     if (arep && !rep_upd[arep[s]]) return;   /* atoms stay inside their replica's range */
-    permute_one(kp, s, src, x, v, mass, kick, pos4, perm, type, tmp_d, tmp4, tmp_i);
+    permute_one(kp, s, src[s], x, v, mass, kick, pos4, perm, type, tmp_d, tmp4, tmp_i);
 }
 
 __global__ void k_copyback(md_kparams kp, const md_devstate *st, int always,
@@ -373,9 +373,9 @@ __device__ __forceinline__ int rebuild_items(int nrep, const md_rep *__restrict_
 }
 
 template <bool BATCH>
-__global__ void __launch_bounds__(CW_WARPS * 32) k_build_cells(
-    md_kparams kp, md_devstate *st, int always, int ncells, int nrep, const float4 *__restrict__ pos4,
-    const int *__restrict__ type, const uint4 *__restrict__ excl_s,
+__global__ void __launch_bounds__(CW_WARPS * 32, 2) k_build_cells(
+    md_kparams kp, md_devstate *st, int always, int ncells, int parts, int any_excl, int nrep,
+    const float4 *__restrict__ pos4, const int *__restrict__ type, const uint4 *__restrict__ excl_s,
     const int *__restrict__ cell_rank, const int *__restrict__ cell_lin,
     const int *__restrict__ cell_start, const unsigned *__restrict__ type_mask, unsigned *nl,
     int *nl_n, float4 *pos_old, const md_rep *__restrict__ reps, const int *__restrict__ crep,
@@ -384,22 +384,25 @@ __global__ void __launch_bounds__(CW_WARPS * 32) k_build_cells(
     pdl_wait();
     pdl_trigger();
     if (!always && !st->update) return;
+    __shared__ build_shm sm;
+    const excl_src ex = {excl_s, nullptr, nullptr, nullptr, any_excl};
     const int lane = threadIdx.x & 31;
     if (BATCH && nrep <= CW_MAXREP) {
         __shared__ int s_pre[CW_MAXREP + 1];
-        const int items = rebuild_items(nrep, reps, rep_upd, s_pre);
+        const int items = rebuild_items(nrep, reps, rep_upd, s_pre) * parts;
         for (;;) {
             int wi = 0;
             if (lane == 0) wi = atomicAdd(&st->cell_next, 1);
             wi = __shfl_sync(0xffffffffu, wi, 0);
             if (wi >= items) break;
-            int lo = 0, hi = nrep;   /* the replica: largest rr with s_pre[rr] <= wi */
+            const int cell = wi / parts;
+            int lo = 0, hi = nrep;   /* the replica: largest rr with s_pre[rr] <= cell */
             while (hi - lo > 1) {
                 const int m = (lo + hi) >> 1;
-                if (s_pre[m] <= wi) lo = m; else hi = m;
+                if (s_pre[m] <= cell) lo = m; else hi = m;
             }
-            build_cell<BATCH>(reps[lo].cell0 + (wi - s_pre[lo]), kp, st, pos4, type, excl_s, cell_rank, cell_lin,
-                              cell_start, type_mask, nl, nl_n, pos_old, reps, crep, rep_upd);
+            build_part<BATCH>(sm, reps[lo].cell0 + (cell - s_pre[lo]), wi - cell * parts, parts, kp, st, pos4, type, ex,
+                              cell_rank, cell_lin, cell_start, type_mask, nl, nl_n, pos_old, reps, crep, rep_upd);
         }
         return;
     }
@@ -407,16 +410,16 @@ __global__ void __launch_bounds__(CW_WARPS * 32) k_build_cells(
         int r = 0;
         if (lane == 0) r = atomicAdd(&st->cell_next, 1);
         r = __shfl_sync(0xffffffffu, r, 0);
-        if (r >= ncells) break;
-        build_cell<BATCH>(r, kp, st, pos4, type, excl_s, cell_rank, cell_lin, cell_start, type_mask, nl,
-                          nl_n, pos_old, reps, crep, rep_upd);
+        if (r >= ncells * parts) break;
+        build_part<BATCH>(sm, r / parts, r % parts, parts, kp, st, pos4, type, ex, cell_rank, cell_lin, cell_start,
+                          type_mask, nl, nl_n, pos_old, reps, crep, rep_upd);
     }
 }
 
 /* The whole rebuild of a single system as one cooperative kernel (the phases
  * of md_rebuild.cuh separated by grid barriers); a launch without a rebuild
  * due returns at once. */
-__global__ void __launch_bounds__(CW_WARPS * 32) k_rebuild_coop(md_kparams kp, md_devstate *st, int always,
+__global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop(md_kparams kp, md_devstate *st, int always,
                                                                 rb_ptrs p)
 {
     /* the same in every block: nothing writes either before the end; a
@@ -454,8 +457,8 @@ static void rb_launch(bool pdl, void (*k)(KArgs...), dim3 grid, dim3 block, cuda
 
 /* Blocks of the persistent warp-per-cell builder: as many as are resident
  * at once (found once per context, on its first, uncaptured, build), at
- * most one warp per cell. */
-static int cw_blocks(md_ctx *c, bool batch)
+ * most one warp per part of a cell (*parts, md_build_parts). */
+static int cw_blocks(md_ctx *c, bool batch, int *parts)
 {
     int &g = c->cw_grid[batch ? 1 : 0];
     if (g == 0) {
@@ -467,7 +470,8 @@ static int cw_blocks(md_ctx *c, bool batch)
         else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_cells<false>, CW_WARPS * 32, 0);
         g = std::max(1, nsm) * std::max(1, occ);
     }
-    return std::max(1, std::min(g, (c->ncells + CW_WARPS - 1) / CW_WARPS));
+    *parts = md_build_parts(c, g * CW_WARPS);
+    return std::max(1, std::min(g, (c->ncells * *parts + CW_WARPS - 1) / CW_WARPS));
 }
 
 /* Whether a single system rebuilds with the one-kernel rebuild: the
@@ -494,7 +498,7 @@ void launch_rebuild(md_ctx *c, const md_kparams &kp, bool unconditional, bool al
     int always = unconditional ? 1 : 0;
     if (c->batch) pdl = false;
     if (md_rebuild_coop(c)) {
-        const rb_ptrs p = make_rb_ptrs(c);
+        const rb_ptrs p = make_rb_ptrs(c, c->coop_grid);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(c->coop_grid);
         cfg.blockDim = dim3(CW_WARPS * 32);
@@ -516,7 +520,8 @@ void launch_rebuild(md_ctx *c, const md_kparams &kp, bool unconditional, bool al
         if (cs != cudaStreamCaptureStatusNone) return;
         c->coop_grid = -1;
     }
-    const int cwb = cw_blocks(c, c->batch);   /* also finds the SM count */
+    int parts = 1;
+    const int cwb = cw_blocks(c, c->batch, &parts);   /* also finds the SM count */
     int nb = (kp.n + 255) / 256;
     cudaStream_t s = c->stream;
     const bool batch = c->batch;
@@ -563,8 +568,8 @@ void launch_rebuild(md_ctx *c, const md_kparams &kp, bool unconditional, bool al
     if (batch) {
         /* at most 5 stencil cells per axis (cells of side >= rl/2): <= 125 */
         k_build_cells<true><<<cwb, CW_WARPS * 32, 0, s>>>(
-            kp, c->st, always, c->ncells, c->nrep, c->pos4, c->type, c->excl_s, c->cell_rank, c->cell_lin,
-            c->cell_start, c->type_mask_dev, c->nl, c->nl_n, c->pos_old, c->reps_dev, c->crep,
+            kp, c->st, always, c->ncells, parts, c->has_bonds, c->nrep, c->pos4, c->type, c->excl_s, c->cell_rank,
+            c->cell_lin, c->cell_start, c->type_mask_dev, c->nl, c->nl_n, c->pos_old, c->reps_dev, c->crep,
             c->rep_upd);
         k_clear_update_b<<<rb, 256, 0, s>>>(c->st, always, c->rep_upd, c->repst, c->nrep);
         return;
@@ -580,7 +585,8 @@ void launch_rebuild(md_ctx *c, const md_kparams &kp, bool unconditional, bool al
     switch (ltpa) {
     case 0:
         rb_launch(pdl, k_build_cells<false>, dim3(cwb),
-                  dim3(CW_WARPS * 32), s, kp, c->st, always, c->ncells, 0, (const float4 *)c->pos4,
+                  dim3(CW_WARPS * 32), s, kp, c->st, always, c->ncells, parts, c->has_bonds, 0,
+                  (const float4 *)c->pos4,
                   (const int *)c->type, (const uint4 *)c->excl_s, (const int *)c->cell_rank,
                   (const int *)c->cell_lin, (const int *)c->cell_start,
                   (const unsigned *)c->type_mask_dev, c->nl, c->nl_n, c->pos_old,

@@ -371,7 +371,6 @@ bool launch_run_steps(md_ctx *c, const md_kparams &kp0, int nsteps)
     md_kparams kp = kp0;
     pair_consts pc = make_pair_consts(c);
     thermo_par tp = make_tp(c, 0);
-    rb_ptrs p = make_rb_ptrs(c);
     run_args a;
     a.st = c->st;
     a.rec = c->rec;
@@ -386,10 +385,11 @@ bool launch_run_steps(md_ctx *c, const md_kparams &kp0, int nsteps)
     a.vir = c->vir;
     a.ljtab = (const float2 *)c->lj_dev;
     a.bonded_par = c->bonded_par;
-    const int na = RUN_THREADS / c->pair_tpa;
+    const int na = RUN_THREADS / c->pair_tpa, blocks = (c->n + na - 1) / na + 1;
+    rb_ptrs p = make_rb_ptrs(c, blocks);
     void *args[] = {&kp, &pc, &tp, &a, &p};
     const void *k = c->lkspace == 0 ? run_kernel<0>(c->pair_tpa) : run_kernel<1>(c->pair_tpa);
-    if (cudaLaunchCooperativeKernel(k, dim3((c->n + na - 1) / na + 1), dim3(RUN_THREADS), args, 0, c->stream) !=
+    if (cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(RUN_THREADS), args, 0, c->stream) !=
         cudaSuccess) {
         (void)cudaGetLastError();
         return false;
