@@ -19,9 +19,12 @@
 namespace {
 
 /* Pair forces of a batch: block b holds 128/TPA atoms of replica tab[b].x
- * starting at tab[b].y. */
+ * starting at tab[b].y.  Bound by issue slots and by the warps that hide the
+ * gathers: at up to two entries per lane, eight blocks per SM at 64
+ * registers (128 replicas of 512 to 8000 ions: 259 us per launch; 277 us at
+ * 72 registers, 312 unbounded, 342 before with one register set and 74). */
 template <int KIND, int TPA, int B, bool ENERGY>
-__global__ void __launch_bounds__(128) k_pair_b(int cap, int pitch, int centered,
+__global__ void __launch_bounds__(128, B <= 2 ? 8 : 1) k_pair_b(int cap, int pitch, int centered,
                                                 const int2 *__restrict__ tab,
                                                 const md_rep *__restrict__ reps,
                                                 const float2 *__restrict__ ljr,
@@ -42,9 +45,7 @@ __global__ void __launch_bounds__(128) k_pair_b(int cap, int pitch, int centered
     __syncthreads();
     const int i = bt.y + (int)threadIdx.x / TPA, lane = (int)threadIdx.x % TPA;
     const bool active = i < end;
-    /* unrolled twice: measured faster here than rolled (1.46 against 1.56 ms
-     * per launch on the 512-replica batch) */
-    pair_total t = pair_sum<KIND, TPA, B, ENERGY, true, 2>(g, cap, active ? i : bt.y, active, lane, pos4,
+    pair_total t = pair_sum<KIND, TPA, B, ENERGY, true, B <= 2 ? 2 : 3>(g, cap, active ? i : bt.y, active, lane, pos4,
                                                   type, nl, nl_n, lj);
     const size_t P = (size_t)pitch;
     if (active && lane == 0) {

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pai
             if (!rebuild_phases(kp, st, p, pos, [&]() { return barrier(0, -1, false, false); })) return;
             load_state();
         }
-        pair_total r = pair_sum<KIND, TPA, B, false, true, 0, false>(geom_kp{kp, pc}, kp.cap, active ? i : 0, active,
+        pair_total r = pair_sum<KIND, TPA, B, false, true, 1, false>(geom_kp{kp, pc}, kp.cap, active ? i : 0, active,
                                                                      lane, pos, p.type, p.nl, p.nl_n, lj);
         if (lane == 0) {
             if (active && (p.has_bonds || p.has_angles)) {

@@ -310,14 +310,22 @@ __device__ __forceinline__ T ld_list(const T *p)
 
 /* The entries of one lane in batches of B, software pipelined: while batch
  * t is computed, the positions of batch t+1 and the list entries of batch
- * t+2 are in flight.  ljrow may point into shared memory (a batch's
- * per-replica table): plain loads there, not the read-only global path. */
-template <int KIND, int TPA, int B, bool ENERGY, bool WRAP, bool PACK, int UNROLL, bool NC, class G>
+ * t+2 are in flight.  SETS = 1 moves them up through one register set in a
+ * rolled loop, SETS = 3 through one unrolled twice; SETS = 2 evaluates two
+ * sets in turn, which saves the moves (6 of 62 instructions per entry) and
+ * costs 16 registers.  Batches take 2 at up to two entries per lane (128
+ * replicas of 512 to 8000 ions: 259 against 342 us per launch unrolled
+ * twice) and 3 above (265 against 285 us at 4 lanes and 4 entries); a single
+ * system's geometry is in the parameter bank and it takes 1 (64000 ions: 43
+ * us with 1, 44.5 with 2, 46 with 3).  ljrow may point into shared memory (a
+ * batch's per-replica table): plain loads there, not the read-only global
+ * path. */
+template <int KIND, int TPA, int B, bool ENERGY, bool WRAP, bool PACK, int SETS, bool NC, class G>
 __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int nb, const unsigned *lp,
                                           const float4 *pos4, const float2 *ljrow, pair_acc &acc)
 {
     unsigned e0[B], e1[B];
-    float4 p0[B];
+    float4 p0[B], p1[B];
     typedef v2<true> V;   /* used when PACK */
     const V PX = V::make(pi.x, pi.x), PY = V::make(pi.y, pi.y), PZ = V::make(pi.z, pi.z);
     const V zero = V::make(0.0f, 0.0f);
@@ -327,42 +335,64 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
     const V PXY = V::make(pi.x, pi.y);
     wrapxy WXY;
     if (!(PACK && !ENERGY && B % 2 == 0) && WRAP) WXY = wrapxy::make(g);
+    auto load_e = [&](unsigned (&e)[B], int t) {
 #pragma unroll
-    for (int b = 0; b < B; b++) e0[b] = ld_list<NC>(lp + b * TPA);
+        for (int b = 0; b < B; b++) e[b] = ld_list<NC>(lp + (t * B + b) * TPA);
+    };
+    auto load_p = [&](float4 (&p)[B], const unsigned (&e)[B]) {
 #pragma unroll
-    for (int b = 0; b < B; b++) p0[b] = ld_list<NC>(pos4 + (e0[b] & MD_INDEX_MASK));
-    if (nb > 1) {
-#pragma unroll
-        for (int b = 0; b < B; b++) e1[b] = ld_list<NC>(lp + (B + b) * TPA);
-    }
-#pragma unroll UNROLL
-    for (int t = 0; t < nb; t++) {
-        float4 p1[B];
-        unsigned e2[B];
-        if (t + 1 < nb) {
-#pragma unroll
-            for (int b = 0; b < B; b++) p1[b] = ld_list<NC>(pos4 + (e1[b] & MD_INDEX_MASK));
-        }
-        if (t + 2 < nb) {
-#pragma unroll
-            for (int b = 0; b < B; b++) e2[b] = ld_list<NC>(lp + ((t + 2) * B + b) * TPA);
-        }
+        for (int b = 0; b < B; b++) p[b] = ld_list<NC>(pos4 + (e[b] & MD_INDEX_MASK));
+    };
+    auto eval = [&](const float4 (&p)[B], const unsigned (&e)[B]) {
         if (PACK && !ENERGY && B % 2 == 0) {
 #pragma unroll
             for (int b = 0; b < B; b += 2)
-                pair_term2<KIND, WRAP, true>(g, W, PX, PY, PZ, qi, p0[b], p0[b + 1], ljrow[e0[b] >> MD_TYPE_SHIFT],
-                                             ljrow[e0[b + 1] >> MD_TYPE_SHIFT], acc2);
+                pair_term2<KIND, WRAP, true>(g, W, PX, PY, PZ, qi, p[b], p[b + 1], ljrow[e[b] >> MD_TYPE_SHIFT],
+                                             ljrow[e[b + 1] >> MD_TYPE_SHIFT], acc2);
         } else {
 #pragma unroll
             for (int b = 0; b < B; b++)
-                pair_term<KIND, ENERGY, WRAP>(g, WXY, PXY, pi, qi, p0[b], ljrow[e0[b] >> MD_TYPE_SHIFT], true,
-                                              acc);
+                pair_term<KIND, ENERGY, WRAP>(g, WXY, PXY, pi, qi, p[b], ljrow[e[b] >> MD_TYPE_SHIFT], true, acc);
         }
+    };
+    load_e(e0, 0);
+    load_p(p0, e0);
+    if (nb > 1) load_e(e1, 1);
+    if (SETS == 2) {
+        /* two register sets in turn, so that no batch is copied from one to
+         * the other: while set 0 is evaluated, set 1's positions and the
+         * entries that replace set 0's are in flight */
+        for (int t = 0;; t += 2) {
+            unsigned e2[B];
+            if (t + 1 < nb) load_p(p1, e1);
+            if (t + 2 < nb) load_e(e2, t + 2);
+            eval(p0, e0);
+            if (t + 1 >= nb) break;
+            if (t + 2 < nb) load_p(p0, e2);
+            unsigned e3[B];
+            if (t + 3 < nb) load_e(e3, t + 3);
+            eval(p1, e1);
+            if (t + 2 >= nb) break;
 #pragma unroll
-        for (int b = 0; b < B; b++) {
-            e0[b] = e1[b];
-            p0[b] = p1[b];
-            e1[b] = e2[b];
+            for (int b = 0; b < B; b++) {
+                e0[b] = e2[b];
+                e1[b] = e3[b];
+            }
+        }
+    } else {
+        constexpr int UNROLL = SETS == 3 ? 2 : 1;
+#pragma unroll UNROLL
+        for (int t = 0; t < nb; t++) {
+            unsigned e2[B];
+            if (t + 1 < nb) load_p(p1, e1);
+            if (t + 2 < nb) load_e(e2, t + 2);
+            eval(p0, e0);
+#pragma unroll
+            for (int b = 0; b < B; b++) {
+                e0[b] = e1[b];
+                p0[b] = p1[b];
+                e1[b] = e2[b];
+            }
         }
     }
     if (PACK && !ENERGY && B % 2 == 0) {
@@ -388,7 +418,7 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
  * FP32 and converts its sum to int64 once; lane sums are combined with
  * integer shuffles (exact), so the result depends only on TPA.  Every lane of
  * the warp must call this (the shuffles use the full mask). */
-template <int KIND, int TPA, int B, bool ENERGY, bool PACK = true, int UNROLL = 0, bool NC = true, class G>
+template <int KIND, int TPA, int B, bool ENERGY, bool PACK = true, int SETS = 1, bool NC = true, class G>
 __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool active, int lane,
                                                const float4 *pos4, const int *type, const unsigned *nl,
                                                const int *nl_n, const float2 *lj)
@@ -396,18 +426,13 @@ __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool
     static_assert(MD_LIST_QUANTUM % (TPA * B) == 0, "batch must divide the list padding");
     const float4 pi = pos4[ii];
     const int cnt = active ? nl_n[ii] : 0;
-    /* unrolling of the batch loop (0: the packed loop rolled, which measured
-     * fastest for a single system, 43 against 46 us per launch on 64000
-     * ions; the scalar one twice) */
-    constexpr int UNR = UNROLL ? UNROLL : ((PACK && !ENERGY && B % 2 == 0) ? 1 : 2);
     /* batches of TPA * B entries up to the first that holds the row's last
      * entry: the row is padded to a multiple of 32 (>= TPA * B) with entries
      * that add exactly zero, so the padding past that batch is skipped.  An
-     * unrolled loop takes whole unrolled rounds where the padding holds
-     * them (an odd count in some of a warp's rows made the unrolled loop's
-     * remainder run as an extra pass: 1.58 against 1.46 ms per launch on the
-     * 512-replica batch) */
-    constexpr int QE = (MD_LIST_QUANTUM % (TPA * B * UNR) == 0) ? TPA * B * UNR : TPA * B;
+     * unrolled loop takes whole unrolled rounds where the padding holds them
+     * (an odd count in some of a warp's rows made its remainder run as an
+     * extra pass: 1.58 against 1.46 ms per launch on 512 replicas) */
+    constexpr int QE = SETS == 3 && MD_LIST_QUANTUM % (TPA * B * 2) == 0 ? TPA * B * 2 : TPA * B;
     const int nb = (cnt + QE - 1) / QE * (QE / (TPA * B));
     const float2 *ljrow = lj + type[ii] * MD_MAXTYPE;
     const float qi = QFAC * pi.w;
@@ -416,9 +441,9 @@ __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool
     const bool inner = g.centered() && __all_sync(0xffffffffu, !active || interior(g, pi));
     if (nb > 0) {
         if (inner)
-            pair_loop<KIND, TPA, B, ENERGY, false, PACK, UNR, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
+            pair_loop<KIND, TPA, B, ENERGY, false, PACK, SETS, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
         else
-            pair_loop<KIND, TPA, B, ENERGY, true, PACK, UNR, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
+            pair_loop<KIND, TPA, B, ENERGY, true, PACK, SETS, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
     }
     pair_total r;
     r.fx = __float2ll_rn(acc.fx * 4294967296.0f);
