@@ -301,8 +301,9 @@ md_status md_set_type_exclusions(md_ctx *ctx, const unsigned *mask);
 /* Arithmetic of the force kernels: 32 (the default) evaluates pair terms in
  * FP32 on the FP32 copy of the positions, as the reference's kernels do
  * (pair_forces.cu:34-205); 64 evaluates pair, bond and angle terms in FP64
- * on the FP64 positions with IEEE sqrt, divide, exp and log (the plain FP64
- * form of the same force law, A&S erfc included).  Forces, integrators and
+ * on the FP64 positions (the plain FP64 form of the same force law, A&S erfc
+ * included; the Coulomb term of pair forces without energies from a
+ * piecewise polynomial within 4e-15 of it).  Forces, integrators and
  * reductions are shared (int64 fixed-point forces, FP64 state).  No
  * counterpart in the reference; the FP64 mode is the GPU reference point of
  * the precision checks.  Recomputes the forces of the current state.  FP64

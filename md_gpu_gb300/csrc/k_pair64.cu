@@ -1,7 +1,10 @@
 /*
  * k_pair64.cu -- the FP64 mode of the force kernels (md_set_precision(ctx,
  * 64)): the same pair and bonded force laws as the FP32 kernels, evaluated
- * in FP64 on the FP64 positions, with IEEE sqrt, divide, exp and log.
+ * in FP64 on the FP64 positions.  Pair forces without energies take the
+ * Coulomb term from a piecewise polynomial within 4e-15 of it and 1/r from
+ * an iteration (rsqrt64); energies and bonded terms use exp, log and IEEE
+ * divide and square root.
  *
  * This is the "plain FP64" form of the path run on the GPU: the reference
  * point of the precision gates (RMS force error, NVE drift) and the per-system
@@ -14,12 +17,13 @@
  * (2^-32 kJ/mol/A: the rounding, ~1e-10 kJ/mol/A, is far below FP32's), so
  * the integrators, thermostats and reductions are shared with the FP32 mode.
  *
- * Layout: 8 lanes per atom, 16 atoms per block of 128 threads; lane l takes
+ * Layout: 8 lanes per atom, 4 or 16 atoms per block; lane l takes
  * the list entries l, l+8, ... of its atom's padded row (the padding entries
  * point at the atom itself, r = 0, and are skipped); each lane sums in FP64,
  * rounds its sums to fixed point once, and the lanes combine with integer
  * shuffles, so the result is deterministic.
  */
+#include <algorithm>
 #include <cstddef>
 #include <cstring>
 
@@ -28,38 +32,71 @@
 namespace {
 
 constexpr int P64_TPA = 8;
-constexpr int P64_THREADS = 128;
-constexpr int P64_ATOMS = P64_THREADS / P64_TPA;
+constexpr int P64_THREADS = 128;   /* per block, at most */
+
+/* What a thread keeps of its md_p64 (the table goes to shared memory). */
+struct md_p64_model {
+    int ni;
+    float nih;
+    double rcsq, rc, rcinv, rc6i, reacf, alpha, spi, pex, a[5], qfac, wolfw, ucc;
+    double L[3], Li[3];
+};
+
+/* 1 / sqrt(s) for s in FP32's normal range: the FP32 approximation and one
+ * step of Halley's iteration, whose error is about e^3 / 3 for a seed of
+ * relative error e / 2 ~ 2^-23; two roundings of the FP64 result remain. */
+__device__ __forceinline__ double rsqrt64(double s, float &seed)
+{
+    seed = rsqrt_approx((float)s);
+    const double y = (double)seed;
+    const double e = fma(-s, y * y, 1.0);
+    return fma(e * y, fma(e, 0.375, 0.5), y);
+}
 
 /* One pair: ff (F_i = ff d) and the pair energy (consistent potential,
- * LJ shifted to zero at rc) for r^2 <= rc^2. */
+ * LJ shifted to zero at rc) for r^2 <= rc^2.  The FP64 pipe issues one warp
+ * instruction in 20 cycles, so its operations are what counts: without
+ * energies the Coulomb term comes from a piecewise polynomial (tab, 8 FP64
+ * operations; exp and the divide of the A&S form take over 40).  4082 ions,
+ * per launch: 230 us before, 102 us now (80% of the FP64 pipe), the error of
+ * eight velocity-Verlet steps against 64 bits unchanged (6.4e-13). */
 template <int KIND, bool ENERGY>
-__device__ __forceinline__ void pair64_eval(const md_p64 &m, double rsq, double qq, double lja,
-                                            double ljc, double &ff, double &u)
+__device__ __forceinline__ void pair64_eval(const md_p64_model &m, const double (*tab)[MD_P64_DEG + 2], double rsq,
+                                            double qq, double lja, double ljc, double &ff, double &u)
 {
-    const double r = sqrt(rsq), ri = 1.0 / r, ri2 = ri * ri;
+    float seed;
+    const double ri = rsqrt64(rsq, seed), r = rsq * ri, ri2 = ri * ri;
     double fc, uc = 0.0;
     if (KIND == 1) {
-        const double xa = m.alpha * r;
-        const double t = 1.0 / (1.0 + m.pex * xa);
-        const double p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
-        const double ex = exp(-xa * xa);
-        const double ec = p * t * ex;
-        fc = qq * ((ec * ri + m.spi * ex) - m.wolfw) * ri2;
-        if (ENERGY) uc = qq * (ec * ri - m.ucc + m.wolfw * log(r * m.rcinv));
+        if (!ENERGY && m.ni > 0) {
+            const double *c = tab[min((int)((float)rsq * seed * m.nih), m.ni - 1)];
+            const double y = r - c[0];
+            double g = c[MD_P64_DEG + 1];
+#pragma unroll
+            for (int k = MD_P64_DEG; k > 0; k--) g = fma(g, y, c[k]);
+            fc = qq * fma(g, ri, -m.wolfw);
+        } else {
+            const double xa = m.alpha * r;
+            const double t = 1.0 / (1.0 + m.pex * xa);
+            const double p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
+            const double ex = exp(-xa * xa);
+            const double ec = p * t * ex;
+            fc = qq * ((ec * ri + m.spi * ex) - m.wolfw);
+            if (ENERGY) uc = qq * (ec * ri - m.ucc + m.wolfw * log(r * m.rcinv));
+        }
     } else {
-        fc = qq * (ri * ri2 - m.reacf);
+        fc = qq * (ri - m.reacf * rsq);
         if (ENERGY) uc = qq * (ri + 0.5 * m.reacf * rsq - m.ucc);
     }
-    const double ri6 = ri2 * ri2 * ri2, ri8 = ri6 * ri2;
-    ff = fc + (lja * ri6 * ri8 - ljc * ri8);
+    const double ri6 = ri2 * ri2 * ri2;
+    ff = ri2 * (fc + ri6 * (lja * ri6 - ljc));
     if (ENERGY)
         u = uc + (lja * (1.0 / 12.0) * (ri6 * ri6 - m.rc6i * m.rc6i) - ljc * (1.0 / 6.0) * (ri6 - m.rc6i));
 }
 
-/* Pair forces in FP64 of a single system (tab == nullptr: block b holds
- * atoms 16b .. 16b+15) or of a batch (block b holds up to 16 atoms of
- * replica tab[b].x from tab[b].y on; geometry, model and LJ table per
+/* Pair forces in FP64 of a single system (tab == nullptr: block b holds the
+ * A = blockDim / 8 atoms from A b on) or of a batch (block b holds up to A
+ * atoms of replica tab[b].x from tab[b].y on; geometry, model and LJ table per
  * replica). */
 template <int KIND, bool ENERGY>
 __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int cap, int centered,
@@ -75,6 +112,7 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
                                                        float *vir, float *epot)
 {
     __shared__ double2 lj[MD_MAXTYPE * MD_MAXTYPE];
+    __shared__ double s_g[MD_P64_MAXI][MD_P64_DEG + 2];
     pdl_trigger();   /* the integrator may be scheduled; it waits for this grid */
     int rep = 0, i0, end;
     if (tab) {
@@ -83,13 +121,38 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
         i0 = bt.y;
         end = reps[rep].atom0 + reps[rep].natom;
     } else {
-        i0 = blockIdx.x * P64_ATOMS;
+        i0 = blockIdx.x * (blockDim.x / P64_TPA);
         end = n;
     }
-    const md_p64 m = models[rep];
-    if (threadIdx.x < MD_MAXTYPE * MD_MAXTYPE) {
-        const float2 l = ljtab[(size_t)rep * MD_MAXTYPE * MD_MAXTYPE + threadIdx.x];
-        lj[threadIdx.x] = make_double2((double)l.x, (double)l.y);
+    md_p64_model m;
+    {
+        const md_p64 &M = models[rep];
+        m.ni = M.ni;
+        m.nih = M.nih;
+        m.rcsq = M.rcsq;
+        m.rc = M.rc;
+        m.rcinv = M.rcinv;
+        m.rc6i = M.rc6i;
+        m.reacf = M.reacf;
+        m.alpha = M.alpha;
+        m.spi = M.spi;
+        m.pex = M.pex;
+        for (int k = 0; k < 5; k++) m.a[k] = M.a[k];
+        m.qfac = M.qfac;
+        m.wolfw = M.wolfw;
+        m.ucc = M.ucc;
+        for (int k = 0; k < 3; k++) {
+            m.L[k] = M.L[k];
+            m.Li[k] = M.Li[k];
+        }
+        if (KIND == 1 && !ENERGY) {
+            const double *g = &M.g[0][0];
+            for (int k = threadIdx.x; k < m.ni * (MD_P64_DEG + 2); k += blockDim.x) (&s_g[0][0])[k] = g[k];
+        }
+    }
+    for (int k = threadIdx.x; k < MD_MAXTYPE * MD_MAXTYPE; k += blockDim.x) {
+        const float2 l = ljtab[(size_t)rep * MD_MAXTYPE * MD_MAXTYPE + k];
+        lj[k] = make_double2((double)l.x, (double)l.y);
     }
     __syncthreads();
     const int i = i0 + (int)threadIdx.x / P64_TPA, lane = (int)threadIdx.x % P64_TPA;
@@ -97,7 +160,9 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
     const int ii = active ? i : i0;
     const size_t P = (size_t)pitch;
     const double xi = x[ii], yi = x[P + ii], zi = x[2 * P + ii];
-    const double qi = m.qfac * (double)pos4[ii].w;
+    const float4 pi = pos4[ii];
+    const float bi[3] = {(float)m.Li[0], (float)m.Li[1], (float)m.Li[2]};
+    const double qi = m.qfac * (double)pi.w;
     const double2 *ljrow = lj + type[ii] * MD_MAXTYPE;
     const int cnt = active ? nl_n[ii] : 0;
     const int npad = (cnt + P64_TPA - 1) / P64_TPA * P64_TPA;   /* padding past it adds zero */
@@ -113,16 +178,26 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
         const unsigned e = __ldg(row + k);
         const int j = (int)(e & MD_INDEX_MASK);
         double dx = xi - x[j], dy = yi - x[P + j], dz = zi - x[2 * P + j];
-        if (!inner) {
+        const float4 pj = pos4[j];
+        if (!inner && centered) {
+            /* the shift's multiple of L from the FP32 positions (it differs
+             * from the FP64 one only for |d| = L/2 to 1e-5 A, beyond rc);
+             * most pairs have none, and then no FP64 operation */
+            const float nx = rint_small((pi.x - pj.x) * bi[0]), ny = rint_small((pi.y - pj.y) * bi[1]),
+                        nz = rint_small((pi.z - pj.z) * bi[2]);
+            if (nx != 0.0f) dx = fma(-m.L[0], (double)nx, dx);
+            if (ny != 0.0f) dy = fma(-m.L[1], (double)ny, dy);
+            if (nz != 0.0f) dz = fma(-m.L[2], (double)nz, dz);
+        } else if (!inner) {
             dx -= m.L[0] * rint(dx * m.Li[0]);
             dy -= m.L[1] * rint(dy * m.Li[1]);
             dz -= m.L[2] * rint(dz * m.Li[2]);
         }
         const double rsq = dx * dx + dy * dy + dz * dz;
-        if (rsq <= m.rcsq && rsq > 0.0) {
+        if (rsq <= m.rcsq && (float)rsq > 0.0f) {
             const double2 l = ljrow[e >> MD_TYPE_SHIFT];
             double ff, u = 0.0;
-            pair64_eval<KIND, ENERGY>(m, rsq, qi * (double)pos4[j].w, l.x, l.y, ff, u);
+            pair64_eval<KIND, ENERGY>(m, s_g, rsq, qi * (double)pj.w, l.x, l.y, ff, u);
             fx += ff * dx;
             fy += ff * dy;
             fz += ff * dz;
@@ -246,6 +321,64 @@ __global__ void k_bonded64(int n, int pitch, const double *__restrict__ boxd,
 
 }  // namespace
 
+/* The pieces of G(r) = E(r) + spi r e^{-a^2 r^2} on [0, rc], E(r) = P5(t) t
+ * e^{-a^2 r^2}, t = 1 / (1 + p a r): on each the Chebyshev interpolant of
+ * degree MD_P64_DEG, written in powers of r - centre.  Takes the fewest
+ * pieces whose largest deviation at 16 points a piece is at most 4e-15 (G is
+ * about 1 or less; FP64 evaluation of the form as written is no closer);
+ * none: m.ni = 0. */
+static void fit_coulomb(md_p64 &m)
+{
+    constexpr int N = MD_P64_DEG + 1;
+    auto G = [&](double r) {
+        const double xa = m.alpha * r, t = 1.0 / (1.0 + m.pex * xa);
+        const double p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
+        const double ex = exp(-xa * xa);
+        return p * t * ex + m.spi * r * ex;
+    };
+    const double pi = 3.14159265358979323846;
+    for (int ni = 16; ni <= MD_P64_MAXI; ni *= 2) {
+        const double h = 0.5 * m.rc / ni;   /* half a piece */
+        double worst = 0.0;
+        for (int q = 0; q < ni; q++) {
+            const double cen = (2 * q + 1) * h;
+            double f[N], mono[N] = {0.0}, tp[N] = {0.0}, tc[N] = {0.0};
+            for (int k = 0; k < N; k++) f[k] = G(cen + h * cos(pi * (k + 0.5) / N));
+            for (int j = 0; j < N; j++) {
+                double a = 0.0;
+                for (int k = 0; k < N; k++) a += f[k] * cos(pi * j * (k + 0.5) / N);
+                a *= (j == 0 ? 1.0 : 2.0) / N;
+                /* tc = T_j in powers: T_0 = 1, T_1 = y, T_j = 2 y T_{j-1} - T_{j-2} */
+                double tn[N] = {0.0};
+                if (j == 0) tn[0] = 1.0;
+                else if (j == 1) tn[1] = 1.0;
+                else
+                    for (int k = 0; k < N; k++) tn[k] = (k > 0 ? 2.0 * tc[k - 1] : 0.0) - tp[k];
+                for (int k = 0; k < N; k++) {
+                    mono[k] += a * tn[k];
+                    tp[k] = tc[k];
+                    tc[k] = tn[k];
+                }
+            }
+            m.g[q][0] = cen;
+            double hk = 1.0;
+            for (int k = 0; k < N; k++, hk *= h) m.g[q][k + 1] = mono[k] / hk;
+            for (int k = 0; k < 16; k++) {
+                const double y = h * (-1.0 + (2 * k + 1) / 16.0);
+                double g = m.g[q][N];
+                for (int d = N - 1; d > 0; d--) g = g * y + m.g[q][d];
+                worst = std::max(worst, fabs(g - G(cen + y)));
+            }
+        }
+        if (worst <= 4e-15) {
+            m.ni = ni;
+            m.nih = (float)(ni / m.rc);
+            return;
+        }
+    }
+    m.ni = 0;
+}
+
 /* FP64 model constants of one system (pairmodel of the plain form): rc from
  * the FP32 rc^2 as given, the Wolf shift and energy constants with the A&S
  * erfc in FP64. */
@@ -283,6 +416,7 @@ md_p64 md_make_p64(int lkspace, float rcutsq, float reacf, float alfa, const flo
     } else if (lkspace == 0) {
         m.ucc = 1.0 / m.rc + 0.5 * m.reacf * m.rcsq;
     }
+    if (lkspace != 0) fit_coulomb(m);
     return m;
 }
 
@@ -290,13 +424,20 @@ void launch_pair64(md_ctx *c, bool energy)
 {
     const bool batch = c->batch != 0;
     const int2 *tab = nullptr;
-    int nb;
+    int dev = 0, nsm = 1, nb;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    /* few atoms: blocks of one warp, so that the SMs' shares of the FP64 work
+     * differ less (4082 ions: 255 blocks of four warps leave some SMs with
+     * two and some with one, 116 us per launch; 102 us with one warp) */
+    const int atoms = c->n / (P64_THREADS / P64_TPA) < 16 * nsm ? 32 / P64_TPA : P64_THREADS / P64_TPA;
+    const int threads = atoms * P64_TPA;
     if (batch) {
-        const int k = md_grid_index(P64_ATOMS);
+        const int k = md_grid_index(atoms);
         tab = c->grid_tab + c->grid_off[k];
         nb = c->grid_cnt[k];
     } else {
-        nb = (c->n + P64_ATOMS - 1) / P64_ATOMS;
+        nb = (c->n + atoms - 1) / atoms;
     }
     const float2 *lj = batch ? c->ljr_dev : (const float2 *)c->lj_dev;
     const md_rep *reps = batch ? c->reps_dev : nullptr;
@@ -305,11 +446,11 @@ void launch_pair64(md_ctx *c, bool energy)
         (const float4 *)c->pos4, (const int *)c->type, (const unsigned *)c->nl, (const int *)c->nl_n, c->f, \
         c->vir, c->epot
     if (c->lkspace == 0) {
-        if (energy) k_pair64<0, true><<<nb, P64_THREADS, 0, c->stream>>>(MD_P64_ARGS);
-        else k_pair64<0, false><<<nb, P64_THREADS, 0, c->stream>>>(MD_P64_ARGS);
+        if (energy) k_pair64<0, true><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
+        else k_pair64<0, false><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
     } else {
-        if (energy) k_pair64<1, true><<<nb, P64_THREADS, 0, c->stream>>>(MD_P64_ARGS);
-        else k_pair64<1, false><<<nb, P64_THREADS, 0, c->stream>>>(MD_P64_ARGS);
+        if (energy) k_pair64<1, true><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
+        else k_pair64<1, false><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
     }
 #undef MD_P64_ARGS
 }

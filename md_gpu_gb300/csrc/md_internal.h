@@ -123,8 +123,15 @@ struct md_rep {
 /* Constants of the FP64 force law of one system or replica (the FP64 mode,
  * md_set_precision): cutoff, reaction-field or Wolf constants, the A&S erfc
  * coefficients widened from the reference's floats, box. */
+constexpr int MD_P64_DEG = 7;     /* degree of a piece of the tabulated Coulomb term */
+constexpr int MD_P64_MAXI = 64;   /* pieces, at most */
 struct md_p64 {
     int kind;   /* lkspace: 0 reaction field, 1 Wolf, 2 LJ + no Coulomb shift */
+    int ni;     /* pieces of G(r) = E(r) + 2 a r / sqrt(pi) e^{-a^2 r^2} on [0, rc], E the A&S
+                   erfc (0: none was accurate enough, G is evaluated as written) */
+    float nih;  /* ni / rc */
+    double g[MD_P64_MAXI][MD_P64_DEG + 2];   /* per piece: its centre, then the coefficients of
+                                                (r - centre)^k */
     double rcsq, rc, rcinv, rc6i, reacf, alpha, spi, pex, a[5], qfac, wolfw, ucc;
     double L[3], Li[3];
 };
