@@ -445,6 +445,7 @@ md_status pme_setup(md_ctx *c, const int K[3])
                 h[((size_t)i * K[1] + j) * (K[2] / 2 + 1) + k] = (float)v;
             }
     MD_CUDA_TRY(c, cudaMemcpy(c->pme.infl, h.data(), sizeof(float) * nspec, cudaMemcpyHostToDevice));
+    MD_CUDA_TRY(c, md_uploads_done());
     /* the neutralising background of a net charge, shared out per atom */
     double qt = 0.0;
     for (int i = 0; i < c->n; i++) qt += (double)c->charge[i];

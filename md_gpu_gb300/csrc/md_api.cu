@@ -443,6 +443,7 @@ md_status initial_build(md_ctx *c)
         if (a != MD_OK) return a;
         int zero = 0;
         MD_CUDA_TRY(c, cudaMemcpy(&c->st->list_overflow, &zero, sizeof(int), cudaMemcpyHostToDevice));
+        MD_CUDA_TRY(c, md_uploads_done());
         kp = md_make_kparams(c);
         launch_rebuild(c, kp, true, true);
         s = check_overflow_and_sync(c);
@@ -654,6 +655,7 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
     if (e == cudaSuccess) e = cudaMemset(c->bl_sn, 0, sizeof(int) * P);
     if (e == cudaSuccess) e = cudaMemset(c->al_sn, 0, sizeof(int) * P);
     if (e == cudaSuccess) e = cudaMemset(c->nl_n, 0, sizeof(int) * P);
+    if (e == cudaSuccess) e = md_uploads_done();
     if (e != cudaSuccess) {
         md_status s = fail(c, MD_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
         md_destroy(c);
@@ -1746,6 +1748,7 @@ static md_status regrid_batch(md_ctx *c)
     MD_CUDA_TRY(c, cudaMemcpy(c->cell_count, zeros.data(), sizeof(int) * cell0, cudaMemcpyHostToDevice));
     MD_CUDA_TRY(c, cudaMemcpy(c->cell_fill, zeros.data(), sizeof(int) * cell0, cudaMemcpyHostToDevice));
     MD_CUDA_TRY(c, cudaMemcpy(c->reps_dev, c->reps.data(), sizeof(md_rep) * c->nrep, cudaMemcpyHostToDevice));
+    MD_CUDA_TRY(c, md_uploads_done());
     for (int k = 0; k < 3; k++) {
         c->ncell[k] = c->reps[0].ncell[k];
         c->binlen[k] = c->reps[0].binlen[k];
@@ -2103,6 +2106,7 @@ md_status md_read_restart(md_ctx *c, const char *path)
     if (r.step > 0)
         MD_CUDA_TRY(c, cudaMemcpy(c->rec + (r.step - 1) % c->rec_cap, &r.last, sizeof(md_thermo),
                                   cudaMemcpyHostToDevice));
+    MD_CUDA_TRY(c, md_uploads_done());
     c->host_step = r.step;
     return MD_OK;
 }
@@ -2336,6 +2340,7 @@ md_status md_set_barostat(md_ctx *c, double press_bar, double tau_p_fs, double c
     c->baro[2] = compressibility_per_bar;
     apply_barostat(c);
     MD_CUDA_TRY(c, cudaMemcpy(c->reps_dev, c->reps.data(), sizeof(md_rep) * c->nrep, cudaMemcpyHostToDevice));
+    MD_CUDA_TRY(c, md_uploads_done());
     return MD_OK;
 }
 
@@ -2375,6 +2380,7 @@ md_status md_debug_list_capacity(md_ctx *c, int capacity, int retry)
         std::vector<int> ones(c->nrep, 1);
         MD_CUDA_TRY(c, cudaMemcpy(c->rep_upd, ones.data(), sizeof(int) * c->nrep, cudaMemcpyHostToDevice));
     }
+    MD_CUDA_TRY(c, md_uploads_done());
     c->overflow_retry = retry ? 1 : 0;
     return MD_OK;
 }
@@ -2401,6 +2407,7 @@ md_status md_set_precision(md_ctx *c, int bits)
         }
         MD_CUDA_TRY(c, dalloc(&c->p64_dev, (size_t)nm));
         MD_CUDA_TRY(c, cudaMemcpy(c->p64_dev, h.data(), sizeof(md_p64) * nm, cudaMemcpyHostToDevice));
+        MD_CUDA_TRY(c, md_uploads_done());
     }
     const int v = bits == 64 ? 1 : 0;
     if (v == c->fp64) return MD_OK;

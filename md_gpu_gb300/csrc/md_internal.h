@@ -346,6 +346,11 @@ md_status pme_setup(md_ctx *c, const int K[3]);
 void pme_free(md_ctx *c);
 /* spread, FFTs, solve and gather of the reciprocal sum, added into the forces */
 void launch_pme(md_ctx *c, const md_kparams &kp, bool energy);
+/* Waits for the copies from pageable memory and the memsets issued so far:
+ * they run on the legacy default stream and may still be under way when the
+ * call returns, and a context's own stream (non-blocking) does not wait for
+ * them.  Call it between such uploads and the launches that read them. */
+inline cudaError_t md_uploads_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
 /* Message returned by md_last_error(NULL, ...). */
 void md_set_global_error(const std::string &msg);
 

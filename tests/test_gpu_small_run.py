@@ -68,3 +68,15 @@ def test_two_small_systems_interleaved():
             a.step(n)
             b.step(n)
         assert np.array_equal(a.positions(), alone[0]) and np.array_equal(b.positions(), alone[1])
+
+
+def test_list_after_creation():
+    """The first list build waits for the uploads and memsets of the creation
+    (they run on another stream): many creations, always the same list."""
+    a = synth.to_arrays(synth.argon_fcc(ncell=7, seed=3, integrator="vv"))
+    counts = []
+    for _ in range(60):
+        with MDSystem.from_arrays(**a) as sim:
+            counts.append(sim.neighbor_list(128)[1])
+    assert counts[0][:1372].min() > 0
+    assert all(np.array_equal(c, counts[0]) for c in counts)
