@@ -375,10 +375,11 @@ md_status md_set_graphs(md_ctx *ctx, int use_graphs);
  * the leapfrog update) as one kernel, 0 as two; MD_ERR_UNSUPPORTED for other
  * systems when asked for 1.  md_autotune times both and keeps the faster. */
 md_status md_set_fused_step(md_ctx *ctx, int fused);
-/* How a step graph holds the neighbour-list rebuild (single systems): 0 (the
- * default) a conditional node per step whose body is the rebuild; 1 the
- * rebuild passes inline in every step, launched as programmatic dependents
- * that return at once when no rebuild is due.  Both rebuild at the same
+/* How a step graph holds the neighbour-list rebuild (single systems): 0 a
+ * conditional node per step whose body is the rebuild; 1 the rebuild inline
+ * in every step, launches that return at once when no rebuild is due.  Until
+ * this, md_set_fused_step or md_autotune is called, systems too large to run
+ * many steps in one launch take 1 (and the fused step where it applies).  Both rebuild at the same
  * steps and give the same trajectory; md_autotune keeps the faster. */
 md_status md_set_graph_rebuild(md_ctx *ctx, int inline_passes);
 /* Milliseconds of device time of the last md_step call (CUDA events). */

@@ -337,8 +337,10 @@ __global__ void __launch_bounds__(256) k_build_list(
  * skip the ones of replicas that keep their lists. */
 constexpr int CW_MAXREP = 4 * CW_WARPS * 32;
 
-__device__ __forceinline__ int rebuild_items(int nrep, const md_rep *__restrict__ reps,
-                                             const int *__restrict__ rep_upd, int *s_pre)
+/* Exclusive prefix sums of of(r), r < nrep <= CW_MAXREP, in s_pre[0 .. nrep]
+ * by a block of CW_WARPS warps; returns the total. */
+template <class F>
+__device__ __forceinline__ int replica_prefix(int nrep, int *s_pre, F &&of)
 {
     constexpr int K = CW_MAXREP / (CW_WARPS * 32);   /* replicas per thread */
     __shared__ int s_wsum[CW_WARPS];
@@ -347,7 +349,7 @@ __device__ __forceinline__ int rebuild_items(int nrep, const md_rep *__restrict_
 #pragma unroll
     for (int k = 0; k < K; k++) {
         const int rr = t * K + k;
-        v[k] = (rr < nrep && rep_upd[rr]) ? reps[rr].ncells : 0;
+        v[k] = rr < nrep ? of(rr) : 0;
         sum += v[k];
     }
     int incl = sum;
@@ -355,6 +357,7 @@ __device__ __forceinline__ int rebuild_items(int nrep, const md_rep *__restrict_
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
     }
+    __syncthreads();   /* s_wsum may still be read by an earlier call */
     if (lane == 31) s_wsum[w] = incl;
     __syncthreads();
     int before = incl - sum, total = 0;
@@ -370,6 +373,17 @@ __device__ __forceinline__ int rebuild_items(int nrep, const md_rep *__restrict_
     }
     __syncthreads();
     return total;
+}
+
+/* The replica whose range of a prefix holds k: the largest r with pre[r] <= k. */
+__device__ __forceinline__ int replica_of(const int *pre, int nrep, int k)
+{
+    int lo = 0, hi = nrep;
+    while (hi - lo > 1) {
+        const int m = (lo + hi) >> 1;
+        if (pre[m] <= k) lo = m; else hi = m;
+    }
+    return lo;
 }
 
 template <bool BATCH>
@@ -389,18 +403,14 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_build_cells(
     const int lane = threadIdx.x & 31;
     if (BATCH && nrep <= CW_MAXREP) {
         __shared__ int s_pre[CW_MAXREP + 1];
-        const int items = rebuild_items(nrep, reps, rep_upd, s_pre) * parts;
+        const int items =
+            replica_prefix(nrep, s_pre, [&](int r) { return rep_upd[r] ? reps[r].ncells : 0; }) * parts;
         for (;;) {
             int wi = 0;
             if (lane == 0) wi = atomicAdd(&st->cell_next, 1);
             wi = __shfl_sync(0xffffffffu, wi, 0);
             if (wi >= items) break;
-            const int cell = wi / parts;
-            int lo = 0, hi = nrep;   /* the replica: largest rr with s_pre[rr] <= cell */
-            while (hi - lo > 1) {
-                const int m = (lo + hi) >> 1;
-                if (s_pre[m] <= cell) lo = m; else hi = m;
-            }
+            const int cell = wi / parts, lo = replica_of(s_pre, nrep, cell);
             build_part<BATCH>(sm, reps[lo].cell0 + (cell - s_pre[lo]), wi - cell * parts, parts, kp, st, pos4, type, ex,
                               cell_rank, cell_lin, cell_start, type_mask, nl, nl_n, pos_old, reps, crep, rep_upd);
         }
@@ -429,6 +439,115 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop(md_kparams kp
     if (*(volatile int *)&st->status != 0) return;
     const unsigned long long bns = p.bar_ns;
     rebuild_phases(kp, st, p, p.pos4, [&]() { return grid_barrier(st, bns); });
+}
+
+/* The rebuild of a batch as one cooperative kernel: the phases of
+ * rebuild_phases over the atoms and cells of the replicas that asked for it
+ * (all: every replica), each replica in its own range of atoms and cells.
+ * Atoms are taken in chunks of 32 of those replicas only.  A launch with no
+ * rebuild due returns at once, so step graphs hold it inline: a conditional
+ * node with the chain of nine passes cost ~10 us a step idle and 80 us per
+ * rebuild of one 7986-ion replica, this kernel 3 and 51 (55 -> 37 us per NPT
+ * step; 607 -> 485 us per step of 128 replicas, 35 of them from here). */
+__global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop_b(
+    md_kparams kp, md_devstate *st, int always, int all, int nrep, rb_ptrs p, const md_rep *__restrict__ reps,
+    const int *__restrict__ crep, int *rep_upd, md_repstate *repst)
+{
+    if (!always && !st->update) return;
+    if (*(volatile int *)&st->status != 0) return;
+    __shared__ build_shm sm;
+    __shared__ int s_pre[CW_MAXREP + 1];   /* cells of the replicas to rebuild before replica r */
+    static_assert(sizeof(build_shm) >= sizeof(int) * (CW_MAXREP + 32 + SCAN_LOCAL + SCAN_LOCAL / SCAN_K),
+                  "chunk prefix and scan buffer");
+    int *chunk = reinterpret_cast<int *>(&sm), *buf = chunk + CW_MAXREP + 32;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31, warp = tid >> 5, warps = nth >> 5, P = kp.pitch;
+    auto bar = [&]() { return grid_barrier(st, p.bar_ns); };
+    const int cells = replica_prefix(nrep, s_pre, [&](int r) { return all || rep_upd[r] ? reps[r].ncells : 0; });
+    const int nch =
+        replica_prefix(nrep, chunk, [&](int r) { return all || rep_upd[r] ? (reps[r].natom + 31) / 32 : 0; });
+    /* every atom of the replicas to rebuild, with its replica */
+    auto for_atoms = [&](auto &&f) {
+        for (int c = warp; c < nch; c += warps) {
+            const int r = replica_of(chunk, nrep, c), a0 = reps[r].atom0;
+            const int i = a0 + (c - chunk[r]) * 32 + lane;
+            if (i < a0 + reps[r].natom) f(i, r);
+        }
+    };
+    int *slot = p.tmp_i + 2 * (size_t)P;
+    for_atoms([&](int i, int r) {
+        const md_rep &R = reps[r];
+        const float4 q = p.pos4[i];
+        const int cx = cell_of(cell_coord(q.x, R.box[0], R.boxi[0], kp.centered), R.box[0], R.binlen[0], R.ncell[0]);
+        const int cy = cell_of(cell_coord(q.y, R.box[1], R.boxi[1], kp.centered), R.box[1], R.binlen[1], R.ncell[1]);
+        const int cz = cell_of(cell_coord(q.z, R.box[2], R.boxi[2], kp.centered), R.box[2], R.binlen[2], R.ncell[2]);
+        const int k = p.cell_rank[R.cell0 + cx + R.ncell[0] * (cy + R.ncell[1] * cz)];
+        p.key[i] = k;
+        slot[i] = atomicAdd(&p.cell_count[k], 1);
+    });
+    if ((int)blockIdx.x == p.bar_drop) return;
+    if (!bar()) return;
+    if (tid == 0) {
+        st->builds += 1;
+        st->cell_next = 0;
+    }
+    /* a block per replica scans its cell counts from its first atom on */
+    for (int r = blockIdx.x; r < nrep; r += gridDim.x) {
+        if (!(all || rep_upd[r])) continue;
+        const int cell0 = reps[r].cell0, nc = reps[r].ncells;
+        int base = reps[r].atom0;
+        for (int c0 = 0; c0 < nc; c0 += SCAN_LOCAL) {
+            const int m = min(SCAN_LOCAL, nc - c0), g0 = cell0 + c0;
+            scan_local(m, p.cell_count + g0, buf);
+            for (int c = threadIdx.x; c < m; c += blockDim.x) p.cell_start[g0 + c] = base + buf[scan_pad(c)];
+            base += buf[scan_pad(m - 1)] + p.cell_count[g0 + m - 1];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) p.cell_start[cell0 + nc] = base;   /* = the next replica's first atom */
+    }
+    if (!bar()) return;
+    for_atoms([&](int i, int) { p.src[p.cell_start[p.key[i]] + slot[i]] = i; });
+    if (!bar()) return;
+    for_atoms([&](int s, int) {
+        const int o = p.src[s], c = p.key[o], mine = p.perm[o];
+        const int b = p.cell_start[c], e = p.cell_start[c + 1];
+        int to = b;
+#pragma unroll 4
+        for (int k = b; k < e; k++) to += p.perm[p.src[k]] < mine ? 1 : 0;
+        permute_one(kp, to, o, p.x, p.v, p.mass, p.kick, p.pos4, p.perm, p.type, p.tmp_d, p.tmp4, p.tmp_i);
+        p.iperm[mine] = to;
+    });
+    for (int k = tid; k < cells; k += nth) {   /* for the next build */
+        const int r = replica_of(s_pre, nrep, k);
+        p.cell_count[reps[r].cell0 + k - s_pre[r]] = 0;
+    }
+    if (!bar()) return;
+    const bool remap = p.has_bonds || p.has_angles;   /* the same in every block */
+    for_atoms([&](int s, int) {
+        copyback_one(kp, s, p.tmp_d, p.tmp4, p.tmp_i, p.x, p.v, p.mass, p.kick, p.pos4, p.perm, nullptr, p.type);
+        if (remap)
+            remap_one(kp, s, p.tmp_i, p.iperm, p.excl_orig, p.excl_s, p.bl_o, p.bl_on, p.bl_s, p.bl_sn, p.al_o,
+                      p.al_on, p.al_s, p.al_sn, p.has_bonds, p.has_angles);
+    });
+    __syncthreads();   /* chunk is overwritten by the list build */
+    const excl_src ex = {p.excl_s, remap ? p.excl_orig : nullptr, p.tmp_i, p.iperm, remap ? 1 : 0};
+    const int items = cells * p.parts;
+    for (int it = warp; it < items;) {
+        const int cell = it / p.parts, r = replica_of(s_pre, nrep, cell);
+        build_part<true>(sm, reps[r].cell0 + cell - s_pre[r], it - cell * p.parts, p.parts, kp, st, p.tmp4, p.tmp_i + P,
+                         ex, p.cell_rank, p.cell_lin, p.cell_start, p.type_mask, p.nl, p.nl_n, p.pos_old, reps, crep,
+                         nullptr);
+        if (items <= warps) break;   /* one item a warp */
+        if (lane == 0) it = warps + atomicAdd(&st->cell_next, 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
+    }
+    if (!bar()) return;
+    for (int r = tid; r < nrep; r += nth)
+        if (all || rep_upd[r]) {
+            repst[r].builds += 1;
+            rep_upd[r] = 0;
+        }
+    if (tid == 0) st->update = 0;
 }
 
 }  // namespace
@@ -474,20 +593,21 @@ static int cw_blocks(md_ctx *c, bool batch, int *parts)
     return std::max(1, std::min(g, (c->ncells * *parts + CW_WARPS - 1) / CW_WARPS));
 }
 
-/* Whether a single system rebuilds with the one-kernel rebuild: the
- * warp-per-cell builder with its stencil in shared memory, and enough
- * resident blocks found for a cooperative launch. */
+/* Whether the context rebuilds with one cooperative kernel: the warp-per-part
+ * builder with its stencil in shared memory, in a batch at most CW_MAXREP
+ * replicas, and enough resident blocks found for a cooperative launch. */
 bool md_rebuild_coop(md_ctx *c)
 {
-    if (c->batch || c->list_tpa != 0 || !c->rebuild_coop) return false;
-    int nst = 1;
+    if (c->list_tpa != 0 || !c->rebuild_coop || (c->batch && c->nrep > CW_MAXREP)) return false;
+    int nst = 1;   /* a batch's stencils have at most 125 cells */
     for (int d = 0; d < 3; d++) nst *= c->stencil[d] < 0 ? c->ncell[d] : 2 * c->stencil[d] + 1;
     if (nst > CW_MAXST) return false;
     if (c->coop_grid == 0) {   /* found once, on the context's first, uncaptured, build */
         int dev = 0, nsm = 0, occ = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rebuild_coop, CW_WARPS * 32, 0);
+        if (c->batch) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rebuild_coop_b, CW_WARPS * 32, 0);
+        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rebuild_coop, CW_WARPS * 32, 0);
         c->coop_grid = occ > 0 ? nsm * occ : -1;
     }
     return c->coop_grid > 0;
@@ -508,7 +628,10 @@ void launch_rebuild(md_ctx *c, const md_kparams &kp, bool unconditional, bool al
         at[0].val.cooperative = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_rebuild_coop, kp, c->st, always, p);
+        const cudaError_t e =
+            c->batch ? cudaLaunchKernelEx(&cfg, k_rebuild_coop_b, kp, c->st, always, all_replicas ? 1 : 0, c->nrep, p,
+                                          (const md_rep *)c->reps_dev, (const int *)c->crep, c->rep_upd, c->repst)
+                     : cudaLaunchKernelEx(&cfg, k_rebuild_coop, kp, c->st, always, p);
         if (e == cudaSuccess) return;
         /* a refused cooperative launch (fewer resident blocks than found
          * when the context was set up) falls back to the chain of passes,

@@ -345,6 +345,11 @@ md_status capture_rebuild_node(md_ctx *c, const md_kparams &kp, cudaGraphConditi
     return MD_OK;
 }
 
+/* Whether step graphs hold the rebuild inline: as chosen for a single
+ * system; in a batch whenever it is one kernel (its chain of passes stays
+ * behind a conditional node). */
+static bool md_inline_rebuild(md_ctx *c) { return c->batch ? md_rebuild_coop(c) : c->rebuild_inline != 0; }
+
 /* A graph of `nsteps` steps.  Each step's rebuild is a conditional node set
  * by the kernel that performed the displacement check, so a step without a
  * rebuild costs only its force and integration kernels. */
@@ -357,8 +362,7 @@ md_status capture_graph(md_ctx *c, int nsteps, int energy_first)
     md_kparams kp = md_make_kparams(c);
     cudaGraph_t g = nullptr;
     MD_CUDA_TRY(c, cudaGraphCreate(&g, 0));
-    /* a batch keeps the conditional node (its passes gate on per-replica flags) */
-    const bool inl = c->rebuild_inline && !c->batch;
+    const bool inl = md_inline_rebuild(c);
     std::vector<cudaGraphConditionalHandle> h(nsteps, 0);
     for (int k = 0; k < (inl ? 0 : nsteps); k++) {
         cudaError_t e = cudaGraphConditionalHandleCreate(&h[k], g, 0, cudaGraphCondAssignDefault);
@@ -449,6 +453,19 @@ md_status initial_build(md_ctx *c)
         s = check_overflow_and_sync(c);
     }
     return s;
+}
+
+/* The form of the step graphs of a single system that nobody chose
+ * (md_autotune, md_set_fused_step, md_set_graph_rebuild): where its steps do
+ * not run in k_run_steps, the one-kernel rebuild inline (64000 ions: an idle
+ * launch 3 us per step, an idle conditional node 10) and, for leapfrog
+ * without bonded terms, pair forces and update as one kernel. */
+void default_step_form(md_ctx *c)
+{
+    if (c->batch || c->form_chosen) return;
+    const int on = !md_can_run_small(c) && md_rebuild_coop(c) ? 1 : 0;
+    c->rebuild_inline = on;
+    c->fuse_step = on;
 }
 
 /* Forces (and KE/T) of the current state, so VV can start and records exist. */
@@ -664,6 +681,7 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
     md_status s = alloc_list(c, (c->nmaxlist + 31) / 32 * 32);
     if (s == MD_OK) s = initial_build(c);
     if (s == MD_OK) s = refresh_state(c);
+    if (s == MD_OK) default_step_form(c);
     if (s != MD_OK) {
         g_last_error = c->last_error;
         md_destroy(c);
@@ -2131,7 +2149,7 @@ md_status md_get_info(md_ctx *c, md_info *out)
     out->pair_entries_per_lane = md_pair_depth(c);
     out->positions_centered = c->centered;
     out->fused_step = md_can_fuse(c) ? 1 : 0;
-    out->rebuild_inline = (c->rebuild_inline && !c->batch) ? 1 : 0;
+    out->rebuild_inline = md_inline_rebuild(c) ? 1 : 0;
     out->list_regrows = c->regrows;
     out->cell_regrids = c->regrids;
     out->list_threads_per_atom = c->list_tpa;
@@ -2146,13 +2164,12 @@ md_status md_get_info(md_ctx *c, md_info *out)
      * the kernels of cuFFT's two transforms, which are not counted */
     if (c->pme.on) out->kernels_per_step += 3 + c->pme.excl;
     for (int k = 0; k < 3; k++) out->pme_grid[k] = c->pme.K[k];
-    /* single system: one cooperative kernel, or key, scan, scatter, order,
-     * permute, copyback, remap (with bonds or angles), list, clear; batch:
-     * flag (forced builds only, not counted), key, scan, scatter, order,
-     * permute, copyback, remap (with bonds or angles), list, clear */
+    /* one cooperative kernel, or key, scan, scatter, order, permute,
+     * copyback, remap (with bonds or angles), list, clear (a batch's forced
+     * builds also flag, not counted) */
     out->kernels_per_rebuild = md_rebuild_coop(c) ? 1 : !(c->has_bonds || c->has_angles) ? 8 : 9;
     out->kernels_per_graph = c->integrator == MD_LEAPFROG ? 1 : 0;
-    if (c->rebuild_inline && !c->batch) {   /* the passes run (and return) in every step */
+    if (md_inline_rebuild(c)) {   /* the passes run (and return) in every step */
         out->kernels_per_step += out->kernels_per_rebuild;
         out->kernels_per_rebuild = 0;
         out->kernels_per_graph = 0;
@@ -2217,6 +2234,7 @@ md_status md_set_pme(md_ctx *c, int k0, int k1, int k2)
     }
     md_status s = pme_setup(c, K);
     if (s != MD_OK) return s;
+    default_step_form(c);
     return refresh_state(c);   /* the forces (and record) of the current state with the new sum */
 }
 
@@ -2233,6 +2251,7 @@ static md_status read_builds(md_ctx *c, int *builds)
 md_status md_autotune(md_ctx *c, int *pair_tpa, int *list_tpa)
 {
     if (!c) return MD_ERR_ARG;
+    c->form_chosen = 1;
     const int lt[] = {0, 4, 8, 16};
     float best = 1e30f;
     int bp = c->pair_tpa, bl = c->list_tpa, bf = 0;
@@ -2416,6 +2435,7 @@ md_status md_set_precision(md_ctx *c, int bits)
         cudaGraphExecDestroy(c->gexec);
         c->gexec = nullptr;
     }
+    default_step_form(c);
     /* the forces (and record) of the current state in the new precision */
     return refresh_state(c);
 }
@@ -2443,6 +2463,7 @@ md_status md_set_graph_rebuild(md_ctx *c, int inline_passes)
 {
     if (!c) return MD_ERR_ARG;
     const int v = inline_passes ? 1 : 0;
+    c->form_chosen = 1;
     if (c->gexec && v != c->rebuild_inline) {
         cudaGraphExecDestroy(c->gexec);
         c->gexec = nullptr;
@@ -2462,6 +2483,7 @@ md_status md_set_fused_step(md_ctx *c, int fused)
                     "md_set_fused_step: only leapfrog single systems without bonded terms fuse");
     }
     c->fuse_step = fused ? 1 : 0;
+    c->form_chosen = 1;
     if (c->gexec && c->fuse_step != old) {
         cudaGraphExecDestroy(c->gexec);
         c->gexec = nullptr;

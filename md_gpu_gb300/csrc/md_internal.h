@@ -250,6 +250,7 @@ struct md_ctx {
     int genergy = 0;
     const float4 *gpos4 = nullptr; /* position buffer current when the graph was captured */
     int use_graphs = 1;            /* 0: launch every step's kernels eagerly */
+    int form_chosen = 0;           /* 1: the caller or the autotuner chose fuse_step, rebuild_inline */
     int fuse_step = 0;             /* 1: fused pair+leapfrog kernel where applicable */
     int cw_grid[2] = {0, 0};       /* blocks of the persistent list builder (single, batch) */
     int rebuild_coop = 1;          /* single systems: the rebuild as one cooperative kernel */

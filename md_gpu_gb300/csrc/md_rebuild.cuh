@@ -335,7 +335,7 @@ __device__ __forceinline__ void build_part(
     cell_geom G;
     if (BATCH) {
         const int rr = crep[r];
-        if (!rep_upd[rr]) return;   /* this replica keeps its list */
+        if (rep_upd && !rep_upd[rr]) return;   /* this replica keeps its list */
         const md_rep &R = reps[rr];
         for (int d = 0; d < 3; d++) {
             G.L[d] = R.box[d]; G.Li[d] = R.boxi[d]; G.nc[d] = R.ncell[d]; G.sten[d] = R.stencil[d];
