@@ -21,10 +21,11 @@ namespace {
 /* Pair forces of a batch: block b holds 128/TPA atoms of replica tab[b].x
  * starting at tab[b].y.  Bound by issue slots and by the warps that hide the
  * gathers: at up to two entries per lane, eight blocks per SM at 64
- * registers (128 replicas of 512 to 8000 ions: 259 us per launch; 277 us at
- * 72 registers, 312 unbounded, 342 before with one register set and 74). */
+ * registers (seven for the reaction field; one register set with energies).
+ * 128 replicas of 512 to 8000 ions: 259 us per launch, 277 us at 72
+ * registers, 312 unbounded, 342 before with one register set and 74. */
 template <int KIND, int TPA, int B, bool ENERGY>
-__global__ void __launch_bounds__(128, B <= 2 ? 8 : 1) k_pair_b(int cap, int pitch, int centered,
+__global__ void __launch_bounds__(128, B > 2 ? 1 : ENERGY || KIND == 1 ? 8 : 7) k_pair_b(int cap, int pitch, int centered,
                                                 const int2 *__restrict__ tab,
                                                 const md_rep *__restrict__ reps,
                                                 const float2 *__restrict__ ljr,
@@ -45,7 +46,7 @@ __global__ void __launch_bounds__(128, B <= 2 ? 8 : 1) k_pair_b(int cap, int pit
     __syncthreads();
     const int i = bt.y + (int)threadIdx.x / TPA, lane = (int)threadIdx.x % TPA;
     const bool active = i < end;
-    pair_total t = pair_sum<KIND, TPA, B, ENERGY, true, B <= 2 ? 2 : 3>(g, cap, active ? i : bt.y, active, lane, pos4,
+    pair_total t = pair_sum<KIND, TPA, B, ENERGY, true, (B > 2 ? 3 : ENERGY ? 1 : 2)>(g, cap, active ? i : bt.y, active, lane, pos4,
                                                   type, nl, nl_n, lj);
     const size_t P = (size_t)pitch;
     if (active && lane == 0) {
@@ -57,14 +58,114 @@ __global__ void __launch_bounds__(128, B <= 2 ? 8 : 1) k_pair_b(int cap, int pit
     }
 }
 
+/* The end of an integrator block of replica rep: as block_close, with the
+ * sums going to the replica's accumulators and a moved atom raising the
+ * replica's rebuild request too.  Returns true in every thread of the last
+ * block to finish.  Thread 0 alone fences: the other threads' stores are
+ * read by later kernels only. */
+__device__ __forceinline__ bool block_close_b(long long a, long long b, long long c, int nsum, bool moved, int rep,
+                                              unsigned long long *racc, int *rep_upd, md_devstate *st,
+                                              unsigned *counter, long long *sh)
+{
+    __shared__ bool last;
+    if (nsum > 0) {
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_down_sync(0xffffffffu, a, o);
+            if (nsum > 1) {
+                b += __shfl_down_sync(0xffffffffu, b, o);
+                c += __shfl_down_sync(0xffffffffu, c, o);
+            }
+        }
+        const int wp = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+        if (l == 0) {
+            sh[wp] = a;
+            sh[nw + wp] = b;
+            sh[2 * nw + wp] = c;
+        }
+    }
+    const int any = __syncthreads_or(moved ? 1 : 0);
+    if (threadIdx.x == 0) {
+        if (nsum > 0) {
+            const int nw = blockDim.x >> 5;
+            long long ta = 0, tb = 0, tc = 0;
+            for (int k = 0; k < nw; k++) {
+                ta += sh[k];
+                tb += sh[nw + k];
+                tc += sh[2 * nw + k];
+            }
+            atomicAdd(racc + 3 * rep, (unsigned long long)ta);
+            if (nsum > 1) {
+                atomicAdd(racc + 3 * rep + 1, (unsigned long long)tb);
+                atomicAdd(racc + 3 * rep + 2, (unsigned long long)tc);
+            }
+        }
+        if (any) {
+            st->update = 1;
+            rep_upd[rep] = 1;
+        }
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return last;
+}
+
+/* Four sums over the block at once (each as block_sum); valid in thread 0. */
+__device__ __forceinline__ void block_sum4(double (&v)[4], double (*sh)[4])
+{
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0)
+#pragma unroll
+        for (int q = 0; q < 4; q++) sh[w][q] = v[q];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = 0.0;
+        for (int k = 0; k < (int)(blockDim.x >> 5); k++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[q] += sh[k][q];
+    }
+}
+
+/* NPT: after a leapfrog step, the replica's box scaled by the factor the
+ * step applied to its positions, and what the kernels derive from it: the
+ * FP32 box and its inverse as the reference rounds it (simulation.cu:
+ * 290-292), 2/L, the wrap limit and the cell side.  The cell grid keeps its
+ * cell counts and stencil until the host lays it out again (md_step does
+ * between chunks of at most 128 steps, before the grid's 3% margin can be
+ * used up at the per-step clamp of mu, 1e-4), so a box whose cells shrink
+ * below half the list radius inside a chunk, or whose list radius exceeds
+ * half the box, can no longer be listed correctly: that sets the sticky
+ * status 2, which the host reports.  Runs in the last block of the step's
+ * leapfrog, when no other block reads the table any more. */
+__device__ void npt_box(md_rep &R, double mu, md_devstate *st)
+{
+    bool bad = false;
+    for (int d = 0; d < 3; d++) {
+        const double L = R.boxd[d] * mu;
+        R.boxd[d] = L;
+        R.box[d] = (float)L;
+        R.boxi[d] = (float)(1.0 / L);
+        R.box2i[d] = 2.0 / L;
+        R.wlim[d] = 0.4999f * R.box[d];
+        R.binlen[d] = R.box[d] / (float)R.ncell[d];
+        if (R.stencil[d] >= 0 && R.binlen[d] < R.rl_half) bad = true;
+        if (2.0f * R.rl_half > 0.5f * R.box[d]) bad = true;
+    }
+    if (bad) atomicOr(&st->status, 2);
+}
+
 /* Runs in the last block to finish: one thread per replica turns its
  * accumulators into KE, PE and virial (and clears them for the next step),
  * then does the replica's thermostat bookkeeping; the batch's step record
  * sums the replicas in a fixed order. */
 __device__ void finalize_b(const md_kparams &kp, const thermo_par &tp, int mode, int nrep,
-                           const md_rep *__restrict__ reps, md_repstate *repst,
-                           unsigned long long *racc, md_devstate *st, md_thermo *rec, int rec_cap,
-                           double *rep_hist, double *sh)
+                           md_rep *reps, md_repstate *repst, unsigned long long *racc, md_devstate *st,
+                           md_thermo *rec, int rec_cap, double *rep_hist, double (*sh)[4])
 {
     double tke = 0.0, tpe = 0.0, tw = 0.0, tex = 0.0;
     /* the step this record belongs to (thread 0 advances it after the sums) */
@@ -72,7 +173,7 @@ __device__ void finalize_b(const md_kparams &kp, const thermo_par &tp, int mode,
     const int builds = ((volatile md_devstate *)st)->builds;
     double *hist = (rep_hist && mode != 2) ? rep_hist + (size_t)(step & (rec_cap - 1)) * 3 * nrep : nullptr;
     for (int r = threadIdx.x; r < nrep; r += blockDim.x) {
-        const md_rep &R = reps[r];
+        md_rep &R = reps[r];
         const double a = fix_take(racc + 3 * r, MD_KFIX);
         double b = fix_take(racc + 3 * r + 1, MD_EFIX);
         double c = fix_take(racc + 3 * r + 2, MD_EFIX);
@@ -86,6 +187,7 @@ __device__ void finalize_b(const md_kparams &kp, const thermo_par &tp, int mode,
             repst[r].pressure = P;
             repst[r].mu_used = repst[r].mu_next;
             repst[r].mu_next = mu;
+            if (R.npt) npt_box(R, repst[r].mu_used, st);
         }
         if (!tp.energy) b = c = 0.0;
         thermo_par t = tp;
@@ -107,11 +209,10 @@ __device__ void finalize_b(const md_kparams &kp, const thermo_par &tp, int mode,
             hist[3 * r + 2] = tp.energy ? ke + b + ex : 0.0;
         }
     }
-    const double KE = block_sum(tke, sh);
-    const double PE = block_sum(tpe, sh);
-    const double W = block_sum(tw, sh);
-    const double EX = block_sum(tex, sh);
+    double tot[4] = {tke, tpe, tw, tex};
+    block_sum4(tot, sh);
     if (threadIdx.x != 0) return;
+    const double KE = tot[0], PE = tot[1], W = tot[2], EX = tot[3];
     st->ke = KE;
     if (tp.energy) {
         st->pe = PE;
@@ -127,7 +228,7 @@ __device__ void finalize_b(const md_kparams &kp, const thermo_par &tp, int mode,
 __global__ void __launch_bounds__(3 * MD_LA) k_leapfrog_b(md_kparams kp, thermo_par tp,
                                                          step_io io, int nrep,
                                                          const int2 *__restrict__ tab,
-                                                         const md_rep *__restrict__ reps,
+                                                         md_rep *reps,
                                                          md_repstate *repst, int *rep_upd,
                                                          unsigned long long *racc,
                                                          double *x, double *v,
@@ -138,7 +239,7 @@ __global__ void __launch_bounds__(3 * MD_LA) k_leapfrog_b(md_kparams kp, thermo_
                                                          const float *__restrict__ epot,
                                                          const float *__restrict__ vir)
 {
-    __shared__ double sh[3 * MD_LA / 32];
+    __shared__ double sh[3 * MD_LA / 32][4];
     __shared__ long long shl[3 * (3 * MD_LA / 32)];
     __shared__ float s_x[3][MD_LA];
     pdl_wait();   /* the forces of this step */
@@ -148,7 +249,7 @@ __global__ void __launch_bounds__(3 * MD_LA) k_leapfrog_b(md_kparams kp, thermo_
     const int s = bt.y + a;
     const bool act = s < R.atom0 + R.natom;
     const size_t o = (size_t)d * kp.pitch + s;
-    double ke2 = 0.0, pe = 0.0, w = 0.0;
+    long long ke = 0, pe = 0, w = 0;
     if (act) {
         axis_par ax = axis_of(d, R.wlim, R.boxd, R.box2i);
         double vv = v[o] + (double)f[o] * kick[s];
@@ -166,21 +267,18 @@ __global__ void __launch_bounds__(3 * MD_LA) k_leapfrog_b(md_kparams kp, thermo_
         }
         s_x[d][a] = wrap(xx, ax.lim, ax.L, ax.two_over_l);
         x[o] = xx;
-        ke2 = mass[s] * (vv * vv);
-        if (d == 0 && tp.energy) pe = epot[s];
-        if (d == 0 && (tp.energy || tp.npt)) w = vir[s];
+        ke = ke_fix(mass[s], vv);
+        if (d == 0 && tp.energy) pe = llrint((double)epot[s] * MD_EFIX);
+        if (d == 0 && (tp.energy || tp.npt)) w = llrint((double)vir[s] * MD_EFIX);
     }
     __syncthreads();
+    bool moved = false;
     if (d == 0 && act) {
         float4 p = make_float4(s_x[0][a], s_x[1][a], s_x[2][a], pos4[s].w);
         pos4[s] = p;
-        if (md_rsq_box(p, io.pos_old[s], R.box, R.boxi) >= R.rmaxdif) {
-            io.st->update = 1;
-            rep_upd[bt.x] = 1;
-        }
+        moved = md_rsq_box(p, io.pos_old[s], R.box, R.boxi) >= R.rmaxdif;
     }
-    block_fix_add(ke2, pe, w, tp.energy || tp.npt, racc + 3 * bt.x, shl);
-    if (md_last_block(io.counter)) {
+    if (block_close_b(ke, pe, w, tp.energy || tp.npt ? 3 : 1, moved, bt.x, racc, rep_upd, io.st, io.counter, shl)) {
         finalize_b(kp, tp, 0, nrep, reps, repst, racc, io.st, io.rec, io.rec_cap, io.rep_hist, sh);
         if (threadIdx.x == 0) {
             set_condition(io);
@@ -218,19 +316,22 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_first_b(md_kparams kp, step_io
         x[o] = xx;
     }
     __syncthreads();
+    bool moved = false;
     if (d == 0 && act) {
         float4 p = make_float4(s_x[0][a], s_x[1][a], s_x[2][a], pos4[s].w);
         pos4[s] = p;
-        if (md_rsq_box(p, io.pos_old[s], R.box, R.boxi) >= R.rmaxdif) {
+        moved = md_rsq_box(p, io.pos_old[s], R.box, R.boxi) >= R.rmaxdif;
+    }
+    if (!io.has_cond) {   /* nothing to do after the last block */
+        if (__syncthreads_or(moved ? 1 : 0) && threadIdx.x == 0) {
             io.st->update = 1;
             rep_upd[bt.x] = 1;
         }
+        return;
     }
-    if (md_last_block(io.counter)) {
-        if (threadIdx.x == 0) {
-            set_condition(io);
-            *io.counter = 0;
-        }
+    if (block_close_b(0, 0, 0, 0, moved, bt.x, nullptr, rep_upd, io.st, io.counter, nullptr) && threadIdx.x == 0) {
+        set_condition(io);
+        *io.counter = 0;
     }
 }
 
@@ -239,8 +340,7 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_first_b(md_kparams kp, step_io
 __global__ void __launch_bounds__(3 * MD_LA) k_vv_second_b(md_kparams kp, thermo_par tp,
                                                           int do_kick, step_io io, int nrep,
                                                           const int2 *__restrict__ tab,
-                                                          const md_rep *__restrict__ reps,
-                                                          md_repstate *repst,
+                                                          md_rep *reps, md_repstate *repst,
                                                           unsigned long long *racc, double *v,
                                                           const double *__restrict__ mass,
                                                           const double *__restrict__ kick,
@@ -248,7 +348,7 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_second_b(md_kparams kp, thermo
                                                           const float *__restrict__ epot,
                                                           const float *__restrict__ vir)
 {
-    __shared__ double sh[3 * MD_LA / 32];
+    __shared__ double sh[3 * MD_LA / 32][4];
     __shared__ long long shl[3 * (3 * MD_LA / 32)];
     pdl_wait();   /* the forces of this step */
     const int2 bt = tab[blockIdx.x];
@@ -256,7 +356,7 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_second_b(md_kparams kp, thermo
     const int d = threadIdx.x / MD_LA, a = threadIdx.x - d * MD_LA;
     const int s = bt.y + a;
     const size_t o = (size_t)d * kp.pitch + s;
-    double ke2 = 0.0, pe = 0.0, w = 0.0;
+    long long ke = 0, pe = 0, w = 0;
     if (s < R.atom0 + R.natom) {
         double vv = v[o];
         if (do_kick) {
@@ -265,47 +365,16 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_second_b(md_kparams kp, thermo
         } else {
             vv *= repst[bt.x].vscale;
         }
-        ke2 = mass[s] * (vv * vv);
-        if (d == 0 && tp.energy) { pe = epot[s]; w = vir[s]; }
+        ke = ke_fix(mass[s], vv);
+        if (d == 0 && tp.energy) {
+            pe = llrint((double)epot[s] * MD_EFIX);
+            w = llrint((double)vir[s] * MD_EFIX);
+        }
     }
-    block_fix_add(ke2, pe, w, tp.energy, racc + 3 * bt.x, shl);
-    if (md_last_block(io.counter)) {
+    if (block_close_b(ke, pe, w, tp.energy ? 3 : 1, false, bt.x, racc, nullptr, io.st, io.counter, shl)) {
         finalize_b(kp, tp, do_kick ? 1 : 2, nrep, reps, repst, racc, io.st, io.rec, io.rec_cap, io.rep_hist, sh);
         if (threadIdx.x == 0) *io.counter = 0;
     }
-}
-
-/* NPT: after a leapfrog step, one thread per replica scales the replica's box
- * by the factor the step applied to its positions (mu_used) and refreshes
- * what the kernels derive from it: the FP32 box and its inverse as the
- * reference rounds it (simulation.cu:290-292), 2/L, the wrap limit and the
- * cell side.  The cell grid keeps its cell counts and stencil until the
- * host lays it out again (md_step does between chunks of at most 128
- * steps, before the grid's 3% margin can be used up at the per-step clamp
- * of mu, 1e-4), so a box whose cells shrink below half the list radius
- * inside a chunk, or whose list radius exceeds half the box, can no longer
- * be listed correctly: that sets the sticky status 2, which the host
- * reports. */
-__global__ void k_npt_box_b(int nrep, md_rep *reps, const md_repstate *__restrict__ repst, md_devstate *st)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrep) return;
-    md_rep &R = reps[r];
-    if (!R.npt) return;
-    const double mu = repst[r].mu_used;
-    bool bad = false;
-    for (int d = 0; d < 3; d++) {
-        const double L = R.boxd[d] * mu;
-        R.boxd[d] = L;
-        R.box[d] = (float)L;
-        R.boxi[d] = (float)(1.0 / L);
-        R.box2i[d] = 2.0 / L;
-        R.wlim[d] = 0.4999f * R.box[d];
-        R.binlen[d] = R.box[d] / (float)R.ncell[d];
-        if (R.stencil[d] >= 0 && R.binlen[d] < R.rl_half) bad = true;
-        if (2.0f * R.rl_half > 0.5f * R.box[d]) bad = true;
-    }
-    if (bad) atomicOr(&st->status, 2);
 }
 
 template <int KIND, bool ENERGY>
@@ -364,23 +433,11 @@ void launch_forces_b(md_ctx *c, const md_kparams &kp, bool energy, int terms)
 void launch_leapfrog_b(md_ctx *c, const md_kparams &kp, int energy, unsigned long long cond,
                        int has_cond)
 {
-    struct npt_after {   /* the box follows the positions the step scaled */
-        md_ctx *c;
-        ~npt_after()
-        {
-            if (c->enstype == 2) launch_npt_box_b(c);
-        }
-    } after{c};
     md_launch_pdl(k_leapfrog_b, dim3(grid_int_blocks(c)), dim3(3 * MD_LA), c->stream, kp,
                   make_tp(c, energy), make_io(c, cond, has_cond), c->nrep, grid_int(c),
-                  (const md_rep *)c->reps_dev, c->repst, c->rep_upd, c->racc, c->x, c->v,
+                  c->reps_dev, c->repst, c->rep_upd, c->racc, c->x, c->v,
                   (const double *)c->mass, (const double *)c->kick, c->pos4,
                   (const long long *)c->f, (const float *)c->epot, (const float *)c->vir);
-}
-
-void launch_npt_box_b(md_ctx *c)
-{
-    k_npt_box_b<<<(c->nrep + 127) / 128, 128, 0, c->stream>>>(c->nrep, c->reps_dev, c->repst, c->st);
 }
 
 void launch_vv_first_b(md_ctx *c, const md_kparams &kp, unsigned long long cond, int has_cond)
@@ -395,7 +452,7 @@ void launch_vv_second_b(md_ctx *c, const md_kparams &kp, int energy, int kick)
 {
     md_launch_pdl(k_vv_second_b, dim3(grid_int_blocks(c)), dim3(3 * MD_LA), c->stream, kp,
                   make_tp(c, energy), kick, make_io(c, 0, 0), c->nrep, grid_int(c),
-                  (const md_rep *)c->reps_dev, c->repst, c->racc, c->v, (const double *)c->mass,
+                  c->reps_dev, c->repst, c->racc, c->v, (const double *)c->mass,
                   (const double *)c->kick, (const long long *)c->f, (const float *)c->epot,
                   (const float *)c->vir);
 }

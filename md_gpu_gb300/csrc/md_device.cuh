@@ -120,18 +120,4 @@ __device__ __forceinline__ void cp_async_wait()
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-/* True in every thread of the block that finishes last (threadfence
- * reduction).  The caller's prior global writes are visible to that block;
- * it must read other blocks' results with __ldcg / volatile and reset the
- * counter. */
-__device__ __forceinline__ bool md_last_block(unsigned *counter)
-{
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    __syncthreads();
-    return last;
-}
-
 #endif

@@ -399,9 +399,6 @@ void launch_leapfrog_b(md_ctx *c, const md_kparams &kp, int energy, unsigned lon
                        int has_cond);
 void launch_vv_first_b(md_ctx *c, const md_kparams &kp, unsigned long long cond, int has_cond);
 void launch_vv_second_b(md_ctx *c, const md_kparams &kp, int energy, int kick);
-/* NPT: every replica's box and cell geometry scaled by the factor its last
- * step applied to its positions (after each leapfrog step of an NPT batch) */
-void launch_npt_box_b(md_ctx *c);
 
 /* List entries each pair-kernel lane loads per batch for the context's
  * lanes per atom: the autotuner's choice, else the default (TPA * depth

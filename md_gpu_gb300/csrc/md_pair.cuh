@@ -193,6 +193,7 @@ __device__ __forceinline__ void pair_term(const G &g, const wrapxy &W, v2<true> 
 template <bool PACKED>
 struct pair_acc2 {
     v2<PACKED> fx, fy, fz, fw;
+    float fe0, fe1;
 };
 
 /* The minimum-image constants as register pairs (the same value in both
@@ -226,8 +227,9 @@ struct wrap2 {
 /* Two pairs (i, j0) and (i, j1) at once: the operations whose operands all
  * vary per entry run on v2; those with a per-atom or per-system constant run
  * as scalar IEEE operations with the constant (no register pair to hold it).
- * The same formulas as pair_term, with every rounding step fixed. */
-template <int KIND, bool WRAP, bool PACKED, class G>
+ * The same formulas as pair_term, with every rounding step fixed, and the
+ * same forces with and without ENERGY. */
+template <int KIND, bool ENERGY, bool WRAP, bool PACKED, class G>
 __device__ __forceinline__ void pair_term2(const G &g, const wrap2<PACKED> &W, v2<PACKED> PX, v2<PACKED> PY,
                                            v2<PACKED> PZ, float qi, float4 p0, float4 p1, float2 l0,
                                            float2 l1, pair_acc2<PACKED> &a)
@@ -244,8 +246,10 @@ __device__ __forceinline__ void pair_term2(const G &g, const wrap2<PACKED> &W, v
     rsq.get(s0, s1);
     const V ri = V::make(rsqrt_approx(s0), rsqrt_approx(s1));
     const V ri2 = ri * ri;
-    const V qq = V::make(__fmul_rn(qi, p0.w), __fmul_rn(qi, p1.w));
+    const float qq0 = __fmul_rn(qi, p0.w), qq1 = __fmul_rn(qi, p1.w);
+    const V qq = V::make(qq0, qq1);
     V ff;
+    float u0 = 0.0f, u1 = 0.0f;   /* Coulomb energy */
     if (KIND == 1) {
         float r0, r1;
         (rsq * ri).get(r0, r1);
@@ -258,10 +262,20 @@ __device__ __forceinline__ void pair_term2(const G &g, const wrap2<PACKED> &W, v
         float h0, h1;
         (h * V::make(e0, e1) * ri).get(h0, h1);
         ff = V::make(__fsub_rn(h0, g.wolf()), __fsub_rn(h1, g.wolf())) * qq;
+        if (ENERGY) {
+            float i0, i1;
+            ri.get(i0, i1);
+            u0 = qq0 * (q0 * e0 * i0 - g.ucc() + g.wolf() * __logf(r0 * g.rcinv()));
+            u1 = qq1 * (q1 * e1 * i1 - g.ucc() + g.wolf() * __logf(r1 * g.rcinv()));
+        }
     } else {
         float a0, a1;
         ri.get(a0, a1);
         ff = qq * V::make(__fmaf_rn(-g.reacf(), s0, a0), __fmaf_rn(-g.reacf(), s1, a1));
+        if (ENERGY) {
+            u0 = qq0 * (a0 + 0.5f * g.reacf() * s0 - g.ucc());
+            u1 = qq1 * (a1 + 0.5f * g.reacf() * s1 - g.ucc());
+        }
     }
     const V ri6 = ri2 * ri2 * ri2;
     float m0, m1;
@@ -271,9 +285,17 @@ __device__ __forceinline__ void pair_term2(const G &g, const wrap2<PACKED> &W, v
     /* list padding entries point at the atom itself: r = 0 is skipped */
     float f0, f1;
     ff.get(f0, f1);
-    f0 = (s0 <= g.rcsq() && s0 > 0.0f) ? f0 : 0.0f;
-    f1 = (s1 <= g.rcsq() && s1 > 0.0f) ? f1 : 0.0f;
+    const bool in0 = s0 <= g.rcsq() && s0 > 0.0f, in1 = s1 <= g.rcsq() && s1 > 0.0f;
+    f0 = in0 ? f0 : 0.0f;
+    f1 = in1 ? f1 : 0.0f;
     ff = V::make(f0, f1);
+    if (ENERGY) {
+        const float c6 = g.rc6i();
+        u0 += l0.x * (1.0f / 12.0f) * (m0 * m0 - c6 * c6) - l0.y * (1.0f / 6.0f) * (m0 - c6);
+        u1 += l1.x * (1.0f / 12.0f) * (m1 * m1 - c6 * c6) - l1.y * (1.0f / 6.0f) * (m1 - c6);
+        a.fe0 += in0 ? 0.5f * u0 : 0.0f;
+        a.fe1 += in1 ? 0.5f * u1 : 0.0f;
+    }
     a.fx = V::fma(ff, dx, a.fx);
     a.fy = V::fma(ff, dy, a.fy);
     a.fz = V::fma(ff, dz, a.fz);
@@ -329,12 +351,12 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
     typedef v2<true> V;   /* used when PACK */
     const V PX = V::make(pi.x, pi.x), PY = V::make(pi.y, pi.y), PZ = V::make(pi.z, pi.z);
     const V zero = V::make(0.0f, 0.0f);
-    pair_acc2<true> acc2 = {zero, zero, zero, zero};
+    pair_acc2<true> acc2 = {zero, zero, zero, zero, 0.0f, 0.0f};
     wrap2<true> W;
     if (PACK && WRAP) W = wrap2<true>::make(g);
     const V PXY = V::make(pi.x, pi.y);
     wrapxy WXY;
-    if (!(PACK && !ENERGY && B % 2 == 0) && WRAP) WXY = wrapxy::make(g);
+    if (!(PACK && B % 2 == 0) && WRAP) WXY = wrapxy::make(g);
     auto load_e = [&](unsigned (&e)[B], int t) {
 #pragma unroll
         for (int b = 0; b < B; b++) e[b] = ld_list<NC>(lp + (t * B + b) * TPA);
@@ -344,10 +366,10 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
         for (int b = 0; b < B; b++) p[b] = ld_list<NC>(pos4 + (e[b] & MD_INDEX_MASK));
     };
     auto eval = [&](const float4 (&p)[B], const unsigned (&e)[B]) {
-        if (PACK && !ENERGY && B % 2 == 0) {
+        if (PACK && B % 2 == 0) {
 #pragma unroll
             for (int b = 0; b < B; b += 2)
-                pair_term2<KIND, WRAP, true>(g, W, PX, PY, PZ, qi, p[b], p[b + 1], ljrow[e[b] >> MD_TYPE_SHIFT],
+                pair_term2<KIND, ENERGY, WRAP, true>(g, W, PX, PY, PZ, qi, p[b], p[b + 1], ljrow[e[b] >> MD_TYPE_SHIFT],
                                              ljrow[e[b + 1] >> MD_TYPE_SHIFT], acc2);
         } else {
 #pragma unroll
@@ -395,7 +417,7 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
             }
         }
     }
-    if (PACK && !ENERGY && B % 2 == 0) {
+    if (PACK && B % 2 == 0) {
         float a0, a1;
         acc2.fx.get(a0, a1);
         acc.fx = __fadd_rn(a0, a1);
@@ -405,14 +427,15 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
         acc.fz = __fadd_rn(a0, a1);
         acc2.fw.get(a0, a1);
         acc.fw = __fadd_rn(a0, a1);
+        acc.fe = acc2.fe0 + acc2.fe1;
     }
 }
 
 /* Pair forces of atom ii from its list: TPA lanes per atom, lane l takes the
  * entries l, l+TPA, ... in batches of B (TPA*B divides 32, the padding
  * quantum of the list rows, so no entry needs a bounds test).  A warp whose
- * atoms are all interior() skips the minimum-image shifts.  With PACK,
- * without energies and with even B, entries go two at a time through
+ * atoms are all interior() skips the minimum-image shifts.  With PACK and
+ * even B, entries go two at a time through
  * pair_term2 as packed f32x2 instructions (each lane keeping even- and
  * odd-entry sums); otherwise one at a time through pair_term.  Each lane sums in
  * FP32 and converts its sum to int64 once; lane sums are combined with

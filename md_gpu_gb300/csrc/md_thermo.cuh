@@ -32,20 +32,6 @@ struct step_io {
     int has_cond;
 };
 
-/* Sum of a double over the block; result valid in thread 0. */
-__device__ __forceinline__ double block_sum(double v, double *sh)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x == 0)
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) r += sh[k];
-    __syncthreads();
-    return r;
-}
-
 /* x -= L trunc(2x/L) (nve_leapfrog.cu:52-56) with 2/L precomputed; returns
  * the FP32 copy of the result.  An atom whose FP32 position lies inside
  * +-0.4999 L is inside +-L/2 in FP64 as well, where trunc gives 0: only atoms
@@ -75,52 +61,15 @@ __device__ __forceinline__ double nh_half_a(double dt, const thermo_par &tp, dou
     return s1;
 }
 
-/* The reductions of a step: each thread's twice-kinetic energy ke2 (m v^2,
- * FP64), potential energy and sum ff r^2 are converted once to fixed point
- * (MD_KFIX = 2^32 per kJ/mol for KE, halved in the same conversion; MD_EFIX
- * = 2^24 for the others) and summed
- * with integer shuffles, shared memory and one atomic add per block and
- * quantity.  Integer addition is exact and associative, so the totals do
- * not depend on the order in which threads or blocks contribute, and the
- * slow FP64 pipe only performs one conversion per thread.  sh holds 3
- * integers per warp. */
-__device__ __forceinline__ void block_fix_add(double ke2, double pe, double w, int energy,
-                                              unsigned long long *acc, long long *sh)
-{
-    long long a = llrint(ke2 * (0.5 * MD_KFIX));
-    long long b = energy ? llrint(pe * MD_EFIX) : 0ll;
-    long long c = energy ? llrint(w * MD_EFIX) : 0ll;
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        if (energy) {
-            b += __shfl_down_sync(0xffffffffu, b, o);
-            c += __shfl_down_sync(0xffffffffu, c, o);
-        }
-    }
-    const int wp = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    if (l == 0) {
-        sh[wp] = a;
-        sh[nw + wp] = b;
-        sh[2 * nw + wp] = c;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long ta = 0, tb = 0, tc = 0;
-        for (int k = 0; k < nw; k++) {
-            ta += sh[k];
-            tb += sh[nw + k];
-            tc += sh[2 * nw + k];
-        }
-        atomicAdd(acc, (unsigned long long)ta);
-        if (energy) {
-            atomicAdd(acc + 1, (unsigned long long)tb);
-            atomicAdd(acc + 2, (unsigned long long)tc);
-        }
-    }
-}
-
+/* The reductions of a step: each thread's kinetic, potential energy and sum
+ * ff r^2 are converted once to fixed point (MD_KFIX = 2^32 per kJ/mol for
+ * KE, MD_EFIX = 2^24 for the others) and summed with integer shuffles,
+ * shared memory and one atomic add per block and quantity.  Integer addition
+ * is exact and associative, so the totals do not depend on the order in
+ * which threads or blocks contribute, and the slow FP64 pipe only performs
+ * one conversion per thread. */
 /* One (atom, axis) kinetic-energy term m v^2 / 2 in 2^-32 kJ/mol fixed
- * point, rounded once (the same value block_fix_add takes from m v^2). */
+ * point, rounded once. */
 __device__ __forceinline__ long long ke_fix(double m, double vv)
 {
     return llrint(m * (vv * vv) * (0.5 * MD_KFIX));
