@@ -437,8 +437,8 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop(md_kparams kp
      * arrival count is then stale) stops every later rebuild */
     if (!always && !st->update) return;
     if (*(volatile int *)&st->status != 0) return;
-    const unsigned long long bns = p.bar_ns;
-    rebuild_phases(kp, st, p, p.pos4, [&]() { return grid_barrier(st, bns); });
+    grid_bar bar = {st, gridDim.x, p.bar_ns, 0ull};
+    if (rebuild_phases(kp, st, p, p.pos4, bar)) bar.arrive_last();
 }
 
 /* The rebuild of a batch as one cooperative kernel: the phases of
@@ -460,12 +460,18 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop_b(
     static_assert(sizeof(build_shm) >= sizeof(int) * (CW_MAXREP + 32 + SCAN_LOCAL + SCAN_LOCAL / SCAN_K),
                   "chunk prefix and scan buffer");
     int *chunk = reinterpret_cast<int *>(&sm), *buf = chunk + CW_MAXREP + 32;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31, warp = tid >> 5, warps = nth >> 5, P = kp.pitch;
-    auto bar = [&]() { return grid_barrier(st, p.bar_ns); };
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = tid >> 5, P = kp.pitch;
     const int cells = replica_prefix(nrep, s_pre, [&](int r) { return all || rep_upd[r] ? reps[r].ncells : 0; });
     const int nch =
         replica_prefix(nrep, chunk, [&](int r) { return all || rep_upd[r] ? (reps[r].natom + 31) / 32 : 0; });
+    /* as many blocks as the work fills, at two atoms or more a warp; the
+     * others leave (the same decision in every block) */
+    const int blocks = min((int)gridDim.x, max(1, nch * 16 / CW_WARPS)), warps = blocks * CW_WARPS;
+    if ((int)blockIdx.x >= blocks) return;
+    const int parts = max(1, min(warps / max(1, cells), (nch * 32 + cells - 1) / max(1, cells)));
+    const int nth = warps * 32;
+    grid_bar bar = {st, (unsigned)blocks, p.bar_ns, 0ull};
     /* every atom of the replicas to rebuild, with its replica */
     auto for_atoms = [&](auto &&f) {
         for (int c = warp; c < nch; c += warps) {
@@ -492,7 +498,7 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop_b(
         st->cell_next = 0;
     }
     /* a block per replica scans its cell counts from its first atom on */
-    for (int r = blockIdx.x; r < nrep; r += gridDim.x) {
+    for (int r = blockIdx.x; r < nrep; r += blocks) {
         if (!(all || rep_upd[r])) continue;
         const int cell0 = reps[r].cell0, nc = reps[r].ncells;
         int base = reps[r].atom0;
@@ -531,23 +537,24 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop_b(
     });
     __syncthreads();   /* chunk is overwritten by the list build */
     const excl_src ex = {p.excl_s, remap ? p.excl_orig : nullptr, p.tmp_i, p.iperm, remap ? 1 : 0};
-    const int items = cells * p.parts;
+    const int items = cells * parts;
     for (int it = warp; it < items;) {
-        const int cell = it / p.parts, r = replica_of(s_pre, nrep, cell);
-        build_part<true>(sm, reps[r].cell0 + cell - s_pre[r], it - cell * p.parts, p.parts, kp, st, p.tmp4, p.tmp_i + P,
+        const int cell = it / parts, r = replica_of(s_pre, nrep, cell);
+        build_part<true>(sm, reps[r].cell0 + cell - s_pre[r], it - cell * parts, parts, kp, st, p.tmp4, p.tmp_i + P,
                          ex, p.cell_rank, p.cell_lin, p.cell_start, p.type_mask, p.nl, p.nl_n, p.pos_old, reps, crep,
                          nullptr);
         if (items <= warps) break;   /* one item a warp */
         if (lane == 0) it = warps + atomicAdd(&st->cell_next, 1);
         it = __shfl_sync(0xffffffffu, it, 0);
     }
-    if (!bar()) return;
-    for (int r = tid; r < nrep; r += nth)
+    if (!bar.arrive_last()) return;
+    /* the last block to finish clears the requests */
+    for (int r = threadIdx.x; r < nrep; r += blockDim.x)
         if (all || rep_upd[r]) {
             repst[r].builds += 1;
             rep_upd[r] = 0;
         }
-    if (tid == 0) st->update = 0;
+    if (threadIdx.x == 0) st->update = 0;
 }
 
 }  // namespace

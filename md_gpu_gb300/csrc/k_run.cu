@@ -69,17 +69,6 @@ struct run_args {
     const float *bonded_par;
 };
 
-__device__ __forceinline__ void red_release(unsigned long long *p)
-{
-    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(1ull) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
-{
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
 template <int KIND, int TPA, int B>
 __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pair_consts pc, thermo_par tp,
                                                               run_args a, rb_ptrs p)
@@ -171,20 +160,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pai
                 if (any) *(volatile unsigned long long *)mv = 1ull;
             }
             red_release(ctl);
-            int ok = 1, it = 0;
-            unsigned long long t0 = 0;
-            while (ld_acquire(ctl) < target) {
-                if ((++it & 127) == 0) {   /* the clock is read now and then */
-                    const unsigned long long now = global_ns();
-                    if (t0 == 0) t0 = now;
-                    else if (now - t0 > bar_ns) {
-                        atomicOr(&st->status, 1);
-                        ok = 0;
-                        break;
-                    }
-                }
-            }
-            s_ok = ok;
+            s_ok = bar_wait(ctl, target, bar_ns, st);
             if (moves) s_flag = *(volatile unsigned long long *)mv != 0ull;
         }
         if (moves) upd_no++;
@@ -241,7 +217,8 @@ __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pai
                 p.x[o] = x;
                 p.v[o] = v;
             }
-            if (!rebuild_phases(kp, st, p, pos, [&]() { return barrier(0, -1, false, false); })) return;
+            auto bar = [&]() { return barrier(0, -1, false, false); };
+            if (!rebuild_phases(kp, st, p, pos, bar) || !bar()) return;
             load_state();
         }
         pair_total r = pair_sum<KIND, TPA, B, false, true, 1, false>(geom_kp{kp, pc}, kp.cap, active ? i : 0, active,

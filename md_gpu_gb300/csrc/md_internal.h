@@ -59,11 +59,9 @@ struct md_devstate {
     unsigned blocks_done; /* blocks finished in the current reduction kernel */
     unsigned long long acc[3]; /* fixed-point KE (MD_KFIX), PE, sum ff r^2 (MD_EFIX) of the step */
     int cell_next;       /* next cell a list-building warp takes (reset after each build) */
-    /* grid barrier of the one-kernel rebuild: arrivals and generation, each
-     * on its own 128-byte line, so that the waiting blocks' polls of the
-     * generation do not contend with the arrivals' atomics */
-    alignas(128) unsigned bar_count;
-    alignas(128) unsigned bar_gen;
+    /* arrivals at the grid barriers of the one-kernel rebuild, on a 128-byte
+     * line of its own; zero between launches */
+    alignas(128) unsigned long long bar_count;
     /* sticky device-side error code (1: a grid barrier timed out), read by
      * the one-kernel rebuild: on a line of its own, which nothing writes
      * unless a wait times out, so those reads never queue behind the

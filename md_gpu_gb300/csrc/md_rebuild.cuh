@@ -649,24 +649,8 @@ __device__ __forceinline__ void build_part(
     }
 }
 
-/* ---- The whole rebuild of a single system as one cooperative kernel ---- */
+/* ---- The whole rebuild as one cooperative kernel ---- */
 
-/* Grid-wide barrier of the cooperative rebuild (every block is resident:
- * the kernel is launched cooperatively).  The last block to arrive resets
- * the count and advances the generation; the others wait for the
- * generation to change for at most bar_ns of global time (MD_BAR_NS unless
- * a test shortens it), after which they record the timeout in st->status.
- * Returns false in every thread of the block when its wait timed out: the
- * caller then returns at once.  A block passes a barrier only when every
- * block has reached it, i.e. after every block finished the phase before
- * it, so no phase runs on counts or prefix sums a barrier did not complete;
- * blocks that passed while another one gave up find that one absent at the
- * next barrier and leave there.  The waiting
- * blocks poll the generation, which lies on another cache line than the
- * arrival counter, so the polls do not slow the arrivals' atomics (the two
- * on one line cost ~12 us per rebuild of 64000 ions with 1216 blocks of 4
- * warps, ~1 us with the 608 blocks of 8 warps used now; a two-level barrier
- * measured no faster). */
 constexpr unsigned long long MD_BAR_NS = 50000000ull;   /* 50 ms */
 
 __device__ __forceinline__ unsigned long long global_ns()
@@ -675,37 +659,84 @@ __device__ __forceinline__ unsigned long long global_ns()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-
-__device__ __forceinline__ bool grid_barrier(md_devstate *st, unsigned long long bar_ns)
+__device__ __forceinline__ void red_release(unsigned long long *p)
 {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *gen = &st->bar_gen;
-        const unsigned g = *gen;
-        __threadfence();
-        int ok = 1;
-        if (atomicAdd(&st->bar_count, 1u) == gridDim.x - 1) {
-            atomicExch(&st->bar_count, 0u);
-            __threadfence();
-            atomicAdd(&st->bar_gen, 1u);
-        } else {
-            const unsigned long long t0 = global_ns();
-            while (*gen == g) {
-                if (global_ns() - t0 > bar_ns) {
-                    atomicOr(&st->status, 1);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(20);
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(1ull) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+/* One thread's wait until *count reaches target: at most bar_ns of global
+ * time, after which it records the timeout in st->status and returns false.
+ * The clock is read now and then. */
+__device__ __forceinline__ bool bar_wait(const unsigned long long *count, unsigned long long target,
+                                         unsigned long long bar_ns, md_devstate *st)
+{
+    int it = 0;
+    unsigned long long t0 = 0;
+    while (ld_acquire(count) < target) {
+        if ((++it & 127) == 0) {
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > bar_ns) {
+                atomicOr(&st->status, 1);
+                return false;
             }
         }
-        __threadfence();
-        s_ok = ok;
     }
-    __syncthreads();
-    return s_ok != 0;
+    return true;
 }
+
+/* Grid-wide barrier of `blocks` blocks that are all resident (a cooperative
+ * launch): each adds one to a count and waits for it to reach the barrier's
+ * multiple of blocks (MD_BAR_NS at most unless a test shortens it).  Returns
+ * false in every thread of the block when its wait timed out: the caller
+ * then returns at once.  A block passes a barrier only when every block has
+ * reached it, i.e. after every block finished the phase before it, so no
+ * phase runs on counts or prefix sums a barrier did not complete; blocks
+ * that passed while another one gave up find that one absent at the next
+ * barrier and leave there.  At the end arrive_last() adds the block without
+ * a wait and returns true in the last one's threads, which then owns what
+ * the kernel leaves for the next launch, the count's reset included.  (A
+ * count and a generation on two lines, with a backoff in the polls, measured
+ * 2 to 3 us more per rebuild.) */
+struct grid_bar {
+    md_devstate *st;
+    unsigned blocks;
+    unsigned long long bar_ns, target;
+    __device__ __forceinline__ bool operator()()
+    {
+        __shared__ int s_ok;
+        __syncthreads();
+        target += blocks;
+        if (threadIdx.x == 0) {
+            red_release(&st->bar_count);
+            s_ok = bar_wait(&st->bar_count, target, bar_ns, st);
+        }
+        __syncthreads();
+        return s_ok != 0;
+    }
+    __device__ __forceinline__ bool arrive_last()
+    {
+        __shared__ int s_last;
+        __syncthreads();
+        target += blocks;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            s_last = atomicAdd(&st->bar_count, 1ull) + 1ull == target;
+            if (s_last) {
+                st->bar_count = 0ull;
+                __threadfence();
+            }
+        }
+        __syncthreads();
+        return s_last != 0;
+    }
+};
 
 /* The arrays the rebuild passes touch. */
 struct rb_ptrs {
@@ -859,8 +890,9 @@ __device__ __forceinline__ void scan_share(int ncells, const int *cell_count, in
 
 /* The rebuild by blocks of CW_WARPS warps (stencils of up to CW_MAXST
  * cells), its phases separated by bar(), a barrier over every block of the
- * grid that returns false when its wait ran out; returns false then.  Ends
- * with a barrier, so the list and the new order are visible to every block.
+ * grid that returns false when its wait ran out; returns false then.  The
+ * list and the new order are visible to every block after the caller's next
+ * barrier.
  *
  *   bin       key and arrival number of every atom in its cell
  *   scan      up to SCAN_LOCAL cells: by every block for itself, with no
@@ -870,7 +902,7 @@ __device__ __forceinline__ void scan_share(int ncells, const int *cell_count, in
  *             the cell's atoms with a smaller original index
  *   build     copy-back, remap and list build, all from the staged order
  *
- * Few barriers (4 with few cells, 5 with many; ~1.3 us each) and parts of
+ * Few barriers (3 with few cells, 4 with many; ~1.3 us each) and parts of
  * cells: a rebuild of a few thousand atoms is bound by latency. */
 template <class Bar>
 __device__ __forceinline__ bool rebuild_phases(const md_kparams &kp, md_devstate *st, const rb_ptrs &p, float4 *pos4,
@@ -934,7 +966,7 @@ __device__ __forceinline__ bool rebuild_phases(const md_kparams &kp, md_devstate
         if (lane == 0) it = (nth >> 5) + atomicAdd(&st->cell_next, 1);
         it = __shfl_sync(0xffffffffu, it, 0);
     }
-    return bar();
+    return true;
 }
 
 }  // namespace
