@@ -132,8 +132,10 @@ md_status md_get_replica_thermo(md_ctx *ctx, md_thermo *out, int nrep);
  * dL/d lj2[a][b] (8x8 per replica, entry a*8+b as used by atoms of type a;
  * the derivative for a symmetric pair parameter is the sum of the (a,b) and
  * (b,a) entries) and dL/d ln s for a common charge scale s, by the discrete
- * adjoint of the integrator with (x, v) checkpoints every `checkpoint` steps
- * and recompute.  The context is left at the end of the trajectory.
+ * adjoint of the integrator, over the positions of every frame when they
+ * take at most a quarter of the device's memory (24 bytes per atom and
+ * frame), else with (x, v) checkpoints every `checkpoint` steps and
+ * recompute.  The context is left at the end of the trajectory.
  * target: nrep*nbins (NULL = 0); loss: nrep; gbar: nrep*nbins (may be NULL);
  * dlj1, dlj2: nrep*64; dlns: nrep. */
 typedef struct {
@@ -368,6 +370,9 @@ md_status md_debug_rebuild_barrier(md_ctx *ctx, double timeout_ms, int drop_bloc
  * a run; retry 0 makes md_step report the overflow (MD_ERR_LIST_OVERFLOW)
  * instead of growing the list and running the steps again. */
 md_status md_debug_list_capacity(md_ctx *ctx, int capacity, int retry);
+/* Test hook (no counterpart in the reference): keep 0 makes md_adjoint_run
+ * run the trajectory again from checkpoints whatever the memory. */
+md_status md_debug_adjoint_frames(md_ctx *ctx, int keep);
 /* md_step launches each step's kernels eagerly instead of replaying a
  * captured graph when use_graphs is 0 (for profilers and debugging). */
 md_status md_set_graphs(md_ctx *ctx, int use_graphs);

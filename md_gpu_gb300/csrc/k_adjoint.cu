@@ -23,11 +23,13 @@
  * atom order, and every sum is taken in a fixed order (block slots, then
  * replicas), so the gradient is deterministic.
  *
- * Checkpoints: (x, v) every C steps in the forward run.  The backward run
- * recomputes one segment of C steps at a time from its checkpoint, keeping
- * its positions, and sweeps the frames of the segment backwards.  Both runs
- * force a list build at every checkpoint frame, so the recomputed
- * trajectory is bit-identical to the forward one.
+ * The forward run keeps the positions of every frame where they fit
+ * (md_adjoint_run), and the backward run sweeps them.  Else checkpoints: (x,
+ * v) every C steps in the forward run; the backward run recomputes one
+ * segment of C steps at a time from its checkpoint, keeping its positions,
+ * and sweeps the frames of the segment backwards.  Both runs force a list
+ * build at every checkpoint frame, so the recomputed trajectory is
+ * bit-identical to the forward one.
  */
 #include <math.h>
 
@@ -149,13 +151,14 @@ __device__ __forceinline__ void rdf_deposit(const adj_par &ap, float r, float wt
     }
 }
 
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_rdf(adj_par ap, const int2 *__restrict__ tab,
+__global__ void __launch_bounds__(ADJ_THREADS, 8) k_adj_rdf(adj_par ap, const int2 *__restrict__ tab,
                                                        const md_rep *__restrict__ reps,
                                                        const float4 *__restrict__ pos4,
                                                        const int *__restrict__ type,
                                                        const unsigned *__restrict__ nl,
                                                        const int *__restrict__ nl_n,
-                                                       unsigned long long *hist)
+                                                       const md_repstate *__restrict__ repst,
+                                                       unsigned long long *hist, double *pe_sum)
 {
     __shared__ unsigned s_h[ADJ_WARPS][ADJ_RDF_BINS];
     __shared__ float s_q[ADJ_WARPS][64];
@@ -164,6 +167,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rdf(adj_par ap, const int2 
     const int2 bt = tab[blockIdx.x];
     const md_rep &R = reps[bt.x];
     const geom_reg g = rep_geom(R);
+    /* the frame's potential energy (from the last velocity-Verlet reduction) */
+    if (threadIdx.x == 0 && (int)blockIdx.x == R.ablk0) pe_sum[bt.x] += repst[bt.x].pe;
     const int a = threadIdx.x / ADJ_TPA, lane = threadIdx.x % ADJ_TPA, w = threadIdx.x >> 5;
     const int wl = threadIdx.x & 31;
     const unsigned lt = (1u << wl) - 1u;
@@ -177,39 +182,47 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rdf(adj_par ap, const int2 
     int cmax = cnt;   /* the warp's longest row */
     for (int o = 16; o > 0; o >>= 1) cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
     int fill = 0;
-    for (int k0 = 0; k0 < cmax; k0 += ADJ_TPA) {
-        const int k = k0 + lane;
-        bool ok = false;
-        float r = 0.0f;
-        if (k < cnt) {
-            const unsigned e = nl[(size_t)i * ap.cap + k];
-            const int j = (int)(e & MD_INDEX_MASK);
-            if ((int)(e >> MD_TYPE_SHIFT) == want && j > i) {
-                const float4 pj = pos4[j];
-                float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                dx -= g.L(0) * rint_small(dx * g.Li(0));
-                dy -= g.L(1) * rint_small(dy * g.Li(1));
-                dz -= g.L(2) * rint_small(dz * g.Li(2));
-                const float rsq = dx * dx + dy * dy + dz * dz;
-                if (rsq < ap.rmaxsq) {
-                    ok = true;
-                    r = rsq * rsqrt_approx(rsq);
-                }
-            }
+    /* RDF_B entries per lane and round, so that their loads are in flight
+     * together (one at a time, a round was a chain of two loads) */
+    constexpr int RDF_B = 4;
+    for (int k0 = 0; k0 < cmax; k0 += ADJ_TPA * RDF_B) {
+        unsigned e[RDF_B];
+        float4 pj[RDF_B];
+        bool ok[RDF_B];
+#pragma unroll
+        for (int b = 0; b < RDF_B; b++) {
+            const int k = k0 + b * ADJ_TPA + lane;
+            e[b] = k < cnt ? nl[(size_t)i * ap.cap + k] : 0u;
+            ok[b] = k < cnt;
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, ok);
-        if (ok) s_q[w][fill + __popc(bal & lt)] = r;
-        fill += __popc(bal);
-        __syncwarp();
-        if (fill >= 32) {
-            rdf_deposit(ap, s_q[w][wl], wt, cstep, s_h[w]);
+#pragma unroll
+        for (int b = 0; b < RDF_B; b++) {
+            const int j = (int)(e[b] & MD_INDEX_MASK);
+            ok[b] = ok[b] && (int)(e[b] >> MD_TYPE_SHIFT) == want && j > i;
+            pj[b] = ok[b] ? pos4[j] : pi;
+        }
+#pragma unroll
+        for (int b = 0; b < RDF_B; b++) {
+            float dx = pi.x - pj[b].x, dy = pi.y - pj[b].y, dz = pi.z - pj[b].z;
+            dx -= g.L(0) * rint_small(dx * g.Li(0));
+            dy -= g.L(1) * rint_small(dy * g.Li(1));
+            dz -= g.L(2) * rint_small(dz * g.Li(2));
+            const float rsq = dx * dx + dy * dy + dz * dz;
+            const bool in = ok[b] && rsq < ap.rmaxsq;
+            const unsigned bal = __ballot_sync(0xffffffffu, in);
+            if (in) s_q[w][fill + __popc(bal & lt)] = rsq * rsqrt_approx(rsq);
+            fill += __popc(bal);
             __syncwarp();
-            const bool mv = wl < fill - 32;
-            const float t = mv ? s_q[w][32 + wl] : 0.0f;
-            __syncwarp();
-            if (mv) s_q[w][wl] = t;
-            fill -= 32;
-            __syncwarp();
+            if (fill >= 32) {
+                rdf_deposit(ap, s_q[w][wl], wt, cstep, s_h[w]);
+                __syncwarp();
+                const bool mv = wl < fill - 32;
+                const float t = mv ? s_q[w][32 + wl] : 0.0f;
+                __syncwarp();
+                if (mv) s_q[w][wl] = t;
+                fill -= 32;
+                __syncwarp();
+            }
         }
     }
     if (wl < fill) rdf_deposit(ap, s_q[w][wl], wt, cstep, s_h[w]);
@@ -221,12 +234,24 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_rdf(adj_par ap, const int2 
     }
 }
 
-/* Per-replica sum of the frame's potential energies (from the last
- * velocity-Verlet reduction), one thread per replica. */
-__global__ void k_adj_pe(int nrep, const md_repstate *__restrict__ repst, double *pe_sum)
+/* A stored frame (original order) as the positions the force kernels read,
+ * and its list check: the replica's request is raised when an atom lies >=
+ * skin/2 from where its list was built. */
+__global__ void k_adj_load(int n, const md_rep *__restrict__ reps, const int *__restrict__ arep,
+                           const int *__restrict__ iperm, const double *__restrict__ frame, float4 *pos4,
+                           const float4 *__restrict__ pos_old, md_devstate *st, int *rep_upd)
 {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nrep) pe_sum[r] += repst[r].pe;
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= n) return;
+    const int s = iperm[o], r = arep[s];
+    const md_rep &R = reps[r];
+    const float4 p = make_float4((float)frame[3 * (size_t)o], (float)frame[3 * (size_t)o + 1],
+                                 (float)frame[3 * (size_t)o + 2], pos4[s].w);
+    pos4[s] = p;
+    if (md_rsq_box(p, pos_old[s], R.box, R.boxi) >= R.rmaxdif) {
+        st->update = 1;
+        rep_upd[r] = 1;
+    }
 }
 
 /* u += dt P (not at the last frame), w = f_m c u with c = dt/(2m) =
@@ -250,18 +275,8 @@ __global__ void k_adj_w(int n, double dt, int update, double fac, const int *__r
     w4[s] = make_float4((float)(c * u[0]), (float)(c * u[1]), (float)(c * u[2]), 0.0f);
 }
 
-/* P += G (sorted-order G, original-order P). */
-__global__ void k_adj_acc(int n, int pitch, const int *__restrict__ perm, const double *__restrict__ G,
-                          double *Pv)
-{
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const size_t o = 3 * (size_t)perm[s];
-    for (int d = 0; d < 3; d++) Pv[o + d] += G[(size_t)d * pitch + s];
-}
-
-/* The bonded part of one frame's adjoint force, added to G after the pair
- * kernel: per sorted atom s, G_s += (J_b w)_s - wpe F_b,s for the harmonic
+/* The bonded part of one frame's adjoint force, added to P after the pair
+ * kernel: per sorted atom s, P_s += (J_b w)_s - wpe F_b,s for the harmonic
  * bonds and angles of k_bonded (bonded_forces.cu:34-193 as the dynamics
  * evaluate them, rsqrtf and acosf included).  (J_b w)_s is the derivative of
  * F_b,s along w: the same expressions carried with their first-order
@@ -279,7 +294,7 @@ __global__ void k_adj_bonded(int n, int pitch, adj_par ap, const md_rep *__restr
                              const float4 *__restrict__ w4, const int2 *__restrict__ bl_s,
                              const int *__restrict__ bl_sn, const int4 *__restrict__ al_s,
                              const int *__restrict__ al_sn, const float *__restrict__ par, int has_bonds,
-                             int has_angles, double *G)
+                             int has_angles, const int *__restrict__ perm, double *Pv)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -353,21 +368,24 @@ __global__ void k_adj_bonded(int n, int pitch, adj_par ap, const md_rep *__restr
         fx += ff * gx; fy += ff * gy; fz += ff * gz;
         tx += ff_t * gx + ff * gx_t; ty += ff_t * gy + ff * gy_t; tz += ff_t * gz + ff * gz_t;
     }
-    G[s] += (double)tx - (double)(wpe * fx);
-    G[(size_t)pitch + s] += (double)ty - (double)(wpe * fy);
-    G[2 * (size_t)pitch + s] += (double)tz - (double)(wpe * fz);
+    double *P = Pv + 3 * (size_t)perm[s];
+    P[0] += (double)tx - (double)(wpe * fx);
+    P[1] += (double)ty - (double)(wpe * fy);
+    P[2] += (double)tz - (double)(wpe * fz);
 }
 
 /* The adjoint pair kernel of one frame: per atom i (ADJ_TPA lanes over its
- * list row) G_i = J(x) w |_i - wpe F_i + d(sum_b e_b g_b)/dx_i, and the
+ * list row) P_i += J(x) w |_i - wpe F_i + d(sum_b e_b g_b)/dx_i, and the
  * row's parameter slots; the block reduces its rows into (type, slot) sums
- * in a fixed order.  ebn[b] = e_b norm_b kn / sigma^2 of the replica. */
+ * in a fixed order and adds them to its own sums over the frames.  Bound by
+ * issue slots and the chain list entry -> position, w; 72 registers keep
+ * seven blocks per SM.  16 x 1000 ions: 75 -> 45 us per frame.  ebn[b] = e_b norm_b kn / sigma^2 of the replica. */
 template <int KIND, int NT>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_back(
+__global__ void __launch_bounds__(ADJ_THREADS, 7) k_adj_back(
     adj_par ap, const int2 *__restrict__ tab, const md_rep *__restrict__ reps,
     const float2 *__restrict__ ljr, const float2 *__restrict__ rtab, const float4 *__restrict__ pos4,
     const int *__restrict__ type, const unsigned *__restrict__ nl, const int *__restrict__ nl_n,
-    const float4 *__restrict__ w4, double *G, double *part)
+    const float4 *__restrict__ w4, const int *__restrict__ perm, double *Pv, double *part)
 {
     constexpr int NS = 2 * NT + 1;           /* slots of a row */
     constexpr int NB = 2 * NT * NT + 1;      /* slots of a block: (type, slot) */
@@ -401,8 +419,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_back(
     sl.ps = 0.f;
     const int cnt = active ? nl_n[ii] : 0;
     const unsigned *row = nl + (size_t)ii * ap.cap;
-    /* the next entry's position and w are loaded while this one is computed */
+    /* the next entry's position and w, and the entry after it, are loaded
+     * while this one is computed */
     unsigned en = lane < cnt ? row[lane] : 0u;
+    unsigned en2 = lane + ADJ_TPA < cnt ? row[lane + ADJ_TPA] : 0u;
     float4 pn = pos4[lane < cnt ? (int)(en & MD_INDEX_MASK) : ii];
     float4 wn = ap.with_w && lane < cnt ? w4[en & MD_INDEX_MASK] : make_float4(0.f, 0.f, 0.f, 0.f);
     for (int k = lane; k < cnt; k += ADJ_TPA) {
@@ -410,10 +430,11 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_back(
         const float4 pj = pn;
         const float4 wj = wn;
         if (k + ADJ_TPA < cnt) {
-            en = row[k + ADJ_TPA];
+            en = en2;
             pn = pos4[en & MD_INDEX_MASK];
             if (ap.with_w) wn = w4[en & MD_INDEX_MASK];
         }
+        if (k + 2 * ADJ_TPA < cnt) en2 = row[k + 2 * ADJ_TPA];
         const int tj = (int)(e >> MD_TYPE_SHIFT);
         float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
         dx -= g.L(0) * rint_small(dx * g.Li(0));
@@ -493,10 +514,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_back(
     }
     if (lane == 0) {
         if (active) {
-            const size_t P = (size_t)ap.pitch;
-            G[i] = gx;
-            G[P + i] = gy;
-            G[2 * P + i] = gz;
+            double *P = Pv + 3 * (size_t)perm[i];
+            P[0] += (double)gx;
+            P[1] += (double)gy;
+            P[2] += (double)gz;
         }
 #pragma unroll
         for (int q = 0; q < NT; q++) {
@@ -519,13 +540,12 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_back(
             for (int r2 = 0; r2 < ADJ_NA; r2++)
                 if (s_type[r2] == tt) acc += (double)s_val[r2][rem];
         }
-        part[(size_t)blockIdx.x * NB + k] = acc;
+        part[(size_t)blockIdx.x * NB + k] += acc;
     }
 }
 
-/* Per replica and block slot (one warp each): the replica's blocks summed
- * lane-strided, then by a fixed shuffle tree, added to its gradient
- * accumulators. */
+/* After the last frame, per replica and block slot (one warp each): the
+ * replica's blocks summed lane-strided, then by a fixed shuffle tree. */
 __global__ void k_adj_param(int nrep, int nb_slots, const md_rep *__restrict__ reps,
                             const double *__restrict__ part, double *acc)
 {
@@ -536,59 +556,62 @@ __global__ void k_adj_param(int nrep, int nb_slots, const md_rep *__restrict__ r
     double s = 0.0;
     for (int b = lane; b < R.anblk; b += 32) s += part[(size_t)(R.ablk0 + b) * nb_slots + k];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) acc[t] += s;
+    if (lane == 0) acc[t] = s;
 }
 
 template <int KIND, int NT>
-void launch_back_nt(md_ctx *c, const adj_par &ap, const float2 *rtab, const float4 *w4, double *G,
+void launch_back_nt(md_ctx *c, const adj_par &ap, const float2 *rtab, const float4 *w4, double *P,
                     double *part)
 {
     const int k = md_grid_index(ADJ_NA);
     k_adj_back<KIND, NT><<<c->grid_cnt[k], ADJ_THREADS, 0, c->stream>>>(
         ap, c->grid_tab + c->grid_off[k], c->reps_dev, c->ljr_dev, rtab, c->pos4, c->type, c->nl,
-        c->nl_n, w4, G, part);
+        c->nl_n, w4, c->perm, P, part);
 }
 
 int adj_nt(int ntype) { return ntype <= 1 ? 1 : (ntype <= 2 ? 2 : (ntype <= 4 ? 4 : 8)); }
 
-void launch_back(md_ctx *c, const adj_par &ap, const float2 *rtab, const float4 *w4, double *G,
+void launch_back(md_ctx *c, const adj_par &ap, const float2 *rtab, const float4 *w4, double *P,
                  double *part)
 {
     const int nt = adj_nt(c->ntype);
 #define MD_ADJ_NT(K, N) \
-    if (c->lkspace == K && nt == N) { launch_back_nt<K == 0 ? 0 : 1, N>(c, ap, rtab, w4, G, part); return; }
+    if (c->lkspace == K && nt == N) { launch_back_nt<K == 0 ? 0 : 1, N>(c, ap, rtab, w4, P, part); return; }
     MD_ADJ_NT(0, 1) MD_ADJ_NT(0, 2) MD_ADJ_NT(0, 4) MD_ADJ_NT(0, 8)
     MD_ADJ_NT(1, 1) MD_ADJ_NT(1, 2) MD_ADJ_NT(1, 4) MD_ADJ_NT(1, 8)
     MD_ADJ_NT(2, 1) MD_ADJ_NT(2, 2) MD_ADJ_NT(2, 4) MD_ADJ_NT(2, 8)
 #undef MD_ADJ_NT
 }
 
-/* Device buffers of one adjoint run. */
+/* Device buffers of one adjoint run, in one allocation. */
 struct adj_buffers {
     double *ck_x = nullptr, *ck_v = nullptr;   /* checkpoints, original order (3n each) */
-    double *seg = nullptr;                     /* positions of one segment's frames */
+    double *seg = nullptr;                     /* positions of one segment's frames, or of all frames */
     double *xK = nullptr, *vK = nullptr;       /* the final state */
-    double *P = nullptr, *U = nullptr, *G = nullptr, *pe_sum = nullptr, *part = nullptr,
-           *acc = nullptr;
+    double *P = nullptr, *U = nullptr, *pe_sum = nullptr, *part = nullptr, *acc = nullptr;
     float4 *w4 = nullptr;
     float *ebn = nullptr;
     float2 *rtab = nullptr;
     unsigned long long *hist = nullptr;
-    ~adj_buffers()
+    char *mem = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T *&p, size_t count)   /* a place in mem (first run: only counted) */
     {
-        void *p[] = {ck_x, ck_v, seg, xK, vK, P, U, G, pe_sum, part, acc, w4, ebn, rtab, hist};
-        for (void *q : p)
-            if (q) cudaFree(q);
+        if (mem) p = (T *)(mem + used);
+        used += (sizeof(T) * std::max<size_t>(count, 1) + 255) / 256 * 256;
     }
+    ~adj_buffers() { cudaFree(mem); }
 };
 
-template <class T>
-cudaError_t adj_alloc(T **p, size_t count)
-{
-    return cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
-}
-
 }  // namespace
+
+extern "C" md_status md_debug_adjoint_frames(md_ctx *c, int keep)
+{
+    if (!c) return MD_ERR_ARG;
+    c->adj_keep = keep ? 1 : 0;
+    return MD_OK;
+}
 
 extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const double *target,
                                     double *loss, double *gbar, double *dlj1, double *dlj2,
@@ -617,23 +640,44 @@ extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const 
     const int nt = adj_nt(c->ntype), NB = 2 * nt * nt + 1;
     const int kla = md_grid_index(ADJ_NA), nblk = c->grid_cnt[kla];
     adj_buffers B;
-    MD_CUDA_TRY(c, adj_alloc(&B.ck_x, 3 * (size_t)n * (nseg + 1)));
-    MD_CUDA_TRY(c, adj_alloc(&B.ck_v, 3 * (size_t)n * (nseg + 1)));
-    MD_CUDA_TRY(c, adj_alloc(&B.seg, 3 * (size_t)n * (C + 1)));
-    MD_CUDA_TRY(c, adj_alloc(&B.xK, 3 * (size_t)n));
-    MD_CUDA_TRY(c, adj_alloc(&B.vK, 3 * (size_t)n));
-    MD_CUDA_TRY(c, adj_alloc(&B.P, 3 * (size_t)n));
-    MD_CUDA_TRY(c, adj_alloc(&B.U, 3 * (size_t)n));
-    MD_CUDA_TRY(c, adj_alloc(&B.G, 3 * (size_t)c->pitch));
-    MD_CUDA_TRY(c, adj_alloc(&B.pe_sum, nrep));
-    MD_CUDA_TRY(c, adj_alloc(&B.part, (size_t)nblk * NB));
-    MD_CUDA_TRY(c, adj_alloc(&B.acc, (size_t)nrep * NB));
-    MD_CUDA_TRY(c, adj_alloc(&B.w4, c->pitch));
-    MD_CUDA_TRY(c, adj_alloc(&B.ebn, (size_t)nrep * nb));
     const float tab_h = (float)(cfg->rdf_dr / 8.0);
     const int tab_n = (int)(rmax / (double)tab_h) + 3;   /* covers [0, rmax + h] */
-    MD_CUDA_TRY(c, adj_alloc(&B.rtab, (size_t)nrep * tab_n));
-    MD_CUDA_TRY(c, adj_alloc(&B.hist, (size_t)nrep * nb));
+    const size_t n3 = 3 * (size_t)n;
+    /* The forward pass keeps every frame's positions when they take at most
+     * a quarter of the device's memory and can be had: the backward pass then
+     * reads them instead of running the trajectory again from checkpoints. */
+    size_t mem_free = 0, mem_total = 0;
+    MD_CUDA_TRY(c, cudaMemGetInfo(&mem_free, &mem_total));
+    bool keep = cfg->gradient && c->adj_keep && sizeof(double) * n3 * (size_t)(K + 1) <= mem_total / 4;
+    auto layout = [&]() {
+        B.used = 0;
+        B.take(B.ck_x, keep || !cfg->gradient ? 0 : n3 * (nseg + 1));
+        B.take(B.ck_v, keep || !cfg->gradient ? 0 : n3 * (nseg + 1));
+        B.take(B.seg, keep ? n3 * (K + 1) : cfg->gradient ? n3 * (C + 1) : 0);
+        B.take(B.xK, n3);
+        B.take(B.vK, n3);
+        B.take(B.P, n3);
+        B.take(B.U, n3);
+        B.take(B.pe_sum, nrep);
+        B.take(B.part, (size_t)nblk * NB);
+        B.take(B.acc, (size_t)nrep * NB);
+        B.take(B.w4, c->pitch);
+        B.take(B.ebn, (size_t)nrep * nb);
+        B.take(B.rtab, (size_t)nrep * tab_n);
+        B.take(B.hist, (size_t)nrep * nb);
+    };
+    layout();
+    cudaError_t ae = cudaMalloc((void **)&B.mem, B.used);
+    if (ae != cudaSuccess && keep) {
+        (void)cudaGetLastError();
+        B.mem = nullptr;
+        keep = false;
+        layout();
+        ae = cudaMalloc((void **)&B.mem, B.used);
+    }
+    if (ae != cudaSuccess) B.mem = nullptr;
+    MD_CUDA_TRY(c, ae);
+    layout();
     cudaStream_t s = c->stream;
     MD_CUDA_TRY(c, cudaMemsetAsync(B.hist, 0, sizeof(unsigned long long) * nrep * nb, s));
     MD_CUDA_TRY(c, cudaMemsetAsync(B.pe_sum, 0, sizeof(double) * nrep, s));
@@ -655,29 +699,23 @@ extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const 
     ap.tab_h = tab_h;
     ap.tab_hi = 1.0f / tab_h;
     ap.tab_n = tab_n;
-    const int rgrid = (nrep + 255) / 256;
     const int agrid = (n + 255) / 256;
 
     md_kparams kp = md_make_kparams(c);
     auto obs = [&]() {
-        k_adj_rdf<<<nblk, ADJ_THREADS, 0, s>>>(ap, c->grid_tab + c->grid_off[kla], c->reps_dev,
-                                                  c->pos4, c->type, c->nl, c->nl_n, B.hist);
-        k_adj_pe<<<rgrid, 256, 0, s>>>(nrep, c->repst, B.pe_sum);
+        k_adj_rdf<<<nblk, ADJ_THREADS, 0, s>>>(ap, c->grid_tab + c->grid_off[kla], c->reps_dev, c->pos4, c->type,
+                                                  c->nl, c->nl_n, c->repst, B.hist, B.pe_sum);
     };
     auto save = [&](double *x, double *v) {
-        launch_gather_out(c, kp, 0, c->io_dev);
-        cudaMemcpyAsync(x, c->io_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s);
-        if (v) {
-            launch_gather_out(c, kp, 1, c->io_dev);
-            cudaMemcpyAsync(v, c->io_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s);
-        }
+        launch_gather_out(c, kp, 0, x);
+        if (v) launch_gather_out(c, kp, 1, v);
     };
     /* one VV step, the list forced at checkpoint frames */
-    auto step = [&](int s_idx) {
+    auto step = [&](int s_idx, bool energy) {   /* the same forces with and without energies */
         launch_vv_first(c, kp, 0, 0);
         launch_rebuild(c, kp, (s_idx + 1) % C == 0, (s_idx + 1) % C == 0);
-        launch_forces(c, kp, true, MD_TERM_ALL);
-        launch_vv_second(c, kp, 1);
+        launch_forces(c, kp, energy, MD_TERM_ALL);
+        launch_vv_second(c, kp, energy ? 1 : 0);
     };
 
     /* ---- forward ---- */
@@ -685,11 +723,16 @@ extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const 
     launch_forces(c, kp, true, MD_TERM_ALL);
     launch_thermo_from_state(c, kp, 1);
     obs();
-    save(B.ck_x, B.ck_v);
+    /* frame m of a kept trajectory, or a checkpoint of one to be run again */
+    auto frame = [&](int m) {
+        if (keep) save(B.seg + n3 * m, nullptr);
+        else if (cfg->gradient && m % C == 0) save(B.ck_x + n3 * (m / C), B.ck_v + n3 * (m / C));
+    };
+    frame(0);
     for (int st = 0; st < K; st++) {
-        step(st);
+        step(st, true);
         obs();
-        if ((st + 1) % C == 0) save(B.ck_x + 3 * (size_t)n * ((st + 1) / C), B.ck_v + 3 * (size_t)n * ((st + 1) / C));
+        frame(st + 1);
     }
     save(B.xK, B.vK);
     std::vector<unsigned long long> hh((size_t)nrep * nb);
@@ -729,41 +772,42 @@ extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const 
     k_adj_rdf_table<<<(nrep * ap.tab_n + 255) / 256, 256, 0, s>>>(ap, nrep, B.ebn, B.rtab);
     MD_CUDA_TRY(c, cudaMemsetAsync(B.P, 0, sizeof(double) * 3 * n, s));
     MD_CUDA_TRY(c, cudaMemsetAsync(B.U, 0, sizeof(double) * 3 * n, s));
-    MD_CUDA_TRY(c, cudaMemsetAsync(B.acc, 0, sizeof(double) * nrep * NB, s));
-    for (int sg = nseg - 1; sg >= 0; sg--) {
+    MD_CUDA_TRY(c, cudaMemsetAsync(B.part, 0, sizeof(double) * (size_t)nblk * NB, s));
+    /* the adjoint of frame m, whose positions are x */
+    auto back = [&](int m, const double *x) {
+        k_adj_load<<<agrid, 256, 0, s>>>(n, c->reps_dev, c->arep, c->iperm, x, c->pos4, c->pos_old, c->st, c->rep_upd);
+        launch_rebuild(c, kp, false, false);
+        ap.with_w = m < K ? 1 : 0;
+        if (m < K)
+            k_adj_w<<<agrid, 256, 0, s>>>(n, (double)c->dt, 1, m >= 1 ? 2.0 : 1.0, c->perm, c->kick, B.U, B.P, B.w4);
+        launch_back(c, ap, B.rtab, B.w4, B.P, B.part);
+        if (c->has_bonds || c->has_angles)
+            k_adj_bonded<<<agrid, 256, 0, s>>>(n, c->pitch, ap, c->reps_dev, c->arep, c->pos4, B.w4, c->bl_s,
+                                                c->bl_sn, c->al_s, c->al_sn, c->bonded_par, c->has_bonds,
+                                                c->has_angles, c->perm, B.P);
+    };
+    if (keep)
+        for (int m = K; m >= 0; m--) back(m, B.seg + n3 * m);
+    /* forces without energies have the same bits where entries are evaluated
+     * two at a time and there are no bonded terms */
+    const bool energy2 = md_pair_depth(c) % 2 != 0 || c->has_bonds || c->has_angles;
+    for (int sg = nseg - 1; sg >= 0 && !keep; sg--) {
         const int m0 = sg * C, m1 = std::min(K, m0 + C);
         /* recompute the segment from its checkpoint, as the forward run did */
-        launch_scatter_in(c, kp, 0, B.ck_x + 3 * (size_t)n * sg);
-        launch_scatter_in(c, kp, 1, B.ck_v + 3 * (size_t)n * sg);
+        launch_scatter_in(c, kp, 0, B.ck_x + n3 * sg);
+        launch_scatter_in(c, kp, 1, B.ck_v + n3 * sg);
         launch_rebuild(c, kp, true, true);
-        launch_forces(c, kp, true, MD_TERM_ALL);
-        MD_CUDA_TRY(c, cudaMemcpyAsync(B.seg, B.ck_x + 3 * (size_t)n * sg, sizeof(double) * 3 * n,
-                                       cudaMemcpyDeviceToDevice, s));
+        launch_forces(c, kp, energy2, MD_TERM_ALL);
+        save(B.seg, nullptr);
         for (int st = m0; st < m1; st++) {
-            step(st);
-            launch_gather_out(c, kp, 0, c->io_dev);
-            MD_CUDA_TRY(c, cudaMemcpyAsync(B.seg + 3 * (size_t)n * (st + 1 - m0), c->io_dev,
-                                           sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s));
+            step(st, energy2);
+            save(B.seg + n3 * (st + 1 - m0), nullptr);
         }
         /* sweep the segment's frames backwards (its last frame belongs to
          * the later segment, except at the end of the trajectory) */
-        for (int m = (m1 == K ? m1 : m1 - 1); m >= m0; m--) {
-            launch_scatter_in(c, kp, 0, B.seg + 3 * (size_t)n * (m - m0));
-            launch_check(c, kp);
-            launch_rebuild(c, kp, false, false);
-            ap.with_w = m < K ? 1 : 0;
-            if (m < K)
-                k_adj_w<<<agrid, 256, 0, s>>>(n, (double)c->dt, 1, m >= 1 ? 2.0 : 1.0, c->perm, c->kick,
-                                               B.U, B.P, B.w4);
-            launch_back(c, ap, B.rtab, B.w4, B.G, B.part);
-            if (c->has_bonds || c->has_angles)
-                k_adj_bonded<<<agrid, 256, 0, s>>>(n, c->pitch, ap, c->reps_dev, c->arep, c->pos4, B.w4, c->bl_s,
-                                                    c->bl_sn, c->al_s, c->al_sn, c->bonded_par, c->has_bonds,
-                                                    c->has_angles, B.G);
-            k_adj_param<<<(nrep * NB * 32 + 255) / 256, 256, 0, s>>>(nrep, NB, c->reps_dev, B.part, B.acc);
-            k_adj_acc<<<agrid, 256, 0, s>>>(n, c->pitch, c->perm, B.G, B.P);
-        }
+        for (int m = (m1 == K ? m1 : m1 - 1); m >= m0; m--) back(m, B.seg + n3 * (m - m0));
     }
+    k_adj_param<<<(nrep * NB * 32 + 255) / 256, 256, 0, s>>>(nrep, NB, c->reps_dev, B.part, B.acc);
     std::vector<double> acc((size_t)nrep * NB);
     MD_CUDA_TRY(c, cudaMemcpyAsync(acc.data(), B.acc, sizeof(double) * acc.size(), cudaMemcpyDeviceToHost, s));
     /* leave the context at the end of the trajectory */

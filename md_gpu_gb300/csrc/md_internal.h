@@ -154,8 +154,9 @@ struct md_repstate {
 #define MD_NGRID 7
 /* Integrator blocks: MD_LA atoms x 3 axes, one thread per (atom, axis). */
 #define MD_LA 128
-/* Atoms per block of the adjoint pair kernels. */
-#define MD_ADJ_ATOMS 32
+/* Atoms per block of the adjoint pair kernels (16 against 32: 45 against 53
+ * us per frame of 16 x 1000 ions, no nearly empty second wave). */
+#define MD_ADJ_ATOMS 16
 /* Fixed-point scales of the energy accumulators: kinetic energy 2^32 per
  * kJ/mol (|KE| < 2.1e9 kJ/mol per system), potential energy and virial 2^24
  * (|PE| < 5.4e11 kJ/mol). */
@@ -301,6 +302,7 @@ struct md_ctx {
     long long snap_host_step = 0;
     int overflow_retry = 1;        /* 0: report a list overflow inside md_step without re-running */
     int regrows = 0;               /* md_step calls re-run after a list overflow */
+    int adj_keep = 1;              /* 0 (test hook): md_adjoint_run recomputes from checkpoints */
     int regrids = 0;               /* NPT: cell grids laid out again for changed boxes */
     md_pme pme;                    /* lkspace 2: the reciprocal Ewald sum (md_set_pme) */
 

@@ -164,6 +164,7 @@ def library(path: Optional[str] = None):
     L.md_set_pme.argtypes = [vp, C.c_int, C.c_int, C.c_int]
     L.md_get_replica_box.argtypes = [vp, vp, vp, C.c_int]
     L.md_debug_list_capacity.argtypes = [vp, C.c_int, C.c_int]
+    L.md_debug_adjoint_frames.argtypes = [vp, C.c_int]
     L.md_get_replica_history.argtypes = [vp, vp, C.c_int, C.POINTER(C.c_int)]
     L.md_set_fused_step.argtypes = [vp, C.c_int]
     L.md_set_graph_rebuild.argtypes = [vp, C.c_int]
