@@ -114,6 +114,8 @@ void launch_forces(md_ctx *c, const md_kparams &kp, bool energy, int terms)
         return;
     }
     pair_consts pc = make_pair_consts(c);
+    const bool recip = c->pme.on && (terms & MD_TERM_RECIP);
+    if (recip) launch_pme_start(c, kp);
     if ((terms & MD_TERM_PAIR) && c->fp64) {
         launch_pair64(c, energy);
     } else if (terms & MD_TERM_PAIR) {
@@ -130,7 +132,7 @@ void launch_forces(md_ctx *c, const md_kparams &kp, bool energy, int terms)
         cudaMemsetAsync(c->epot, 0, sizeof(float) * (size_t)c->pitch, c->stream);
     }
     launch_bonded(c, kp, energy, terms);
-    if (c->pme.on && (terms & MD_TERM_RECIP)) launch_pme(c, kp, energy);
+    if (recip) launch_pme_finish(c, kp, energy);
 }
 
 void launch_bonded(md_ctx *c, const md_kparams &kp, bool energy, int terms)

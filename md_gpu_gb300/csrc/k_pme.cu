@@ -111,131 +111,141 @@ __global__ void k_pme_prep(pme_par pp, const double *__restrict__ x, const float
     wq[s] = make_float4(w[0], w[1], w[2], pos4[s].w);
 }
 
-/* Charge grid, one block per brick (see the file comment).  The block
- * walks the candidate atoms 256 at a time: each thread tests one and
- * queues it (spline origin relative to the brick, its 12 weights, charge)
- * when its spline reaches the brick; then the block's threads take the
- * queued atoms' 64 (atom, point) products one each, so every lane adds one
- * grid point per pass instead of one thread looping over an atom's 64. */
+/* Charge grid, one block per brick (see the file comment).  Half-warps take
+ * the candidate cells (those that overlap this brick's window; their atom
+ * ranges are loaded first, by all threads at once), 16 atoms at a time, and
+ * queue each atom whose spline reaches the brick (spline origin relative to
+ * the brick, its 12 weights, charge).  A queue that might not hold the next
+ * round, and the last one, is deposited: each lane adds one (atom, x, y) row
+ * of four z points per pass.  Bound by latency, so few rounds and few
+ * barriers count, and few instructions: 64000 ions, 112^3, per launch 32 us
+ * with a prefix sum by one warp, a search per candidate, the 64 cells of the
+ * widest brick, a deposit per 256 candidates and 64-bit conversions; 25 us
+ * so. */
+constexpr int PQ = 384;   /* queue slots */
+/* strides of the brick's points in shared memory: the 4 x 4 rows of an atom,
+ * which one half-warp adds to at once, begin in 16 different banks */
+constexpr int SY = PB + 1, SX = PB * SY + 2;
 __global__ void __launch_bounds__(256) k_pme_spread(pme_par pp, const int4 *__restrict__ org,
                                                     const float4 *__restrict__ wq,
                                                     const int *__restrict__ cell_rank,
                                                     const int *__restrict__ cell_start, float *grid)
 {
     /* the 2^-32 fixed-point sum of a grid point as two 32-bit sums (native
-     * shared-memory atomics): v = hi 2^20 + lo with lo = v mod 2^20; lo
-     * sums stay exact for up to 2048 contributions per point, hi for
-     * charges below 256 e */
-    __shared__ int s_hi[PB * PB * PB];
-    __shared__ int s_lo[PB * PB * PB];
-    __shared__ int s_start[PME_MAXC * PME_MAXC * PME_MAXC];   /* first atom of each candidate cell */
-    __shared__ int s_pre[PME_MAXC * PME_MAXC * PME_MAXC + 1];
-    __shared__ int s_rel[256];          /* queued atom: (rx, ry, rz) packed 8 bits each */
-    __shared__ float s_th[256][13];     /* queued atom: x, y, z weights (4 each) and charge */
+     * shared-memory atomics): v = hi 2^20 + lo with |lo| <= 2^19; lo sums
+     * stay exact for up to 4096 contributions per point, hi for weighted
+     * charges below 512 e */
+    __shared__ int s_hi[PB * SX];
+    __shared__ int s_lo[PB * SX];
+    __shared__ int2 s_cell[PME_MAXC * PME_MAXC * PME_MAXC];   /* atom range of each candidate cell */
+    __shared__ int s_rel[PQ];          /* queued atom: (rx, ry, rz) packed 8 bits each */
+    __shared__ __align__(16) float s_th[PQ][12];   /* queued atom: q x, y and z weights (4 each) */
     __shared__ int s_nq;
     const int tid = threadIdx.x;
     const int nbz = pp.K[2] / PB, nby = pp.K[1] / PB;
     const int bz = blockIdx.x % nbz, by = (blockIdx.x / nbz) % nby, bx = blockIdx.x / (nbz * nby);
     const int lo[3] = {bx * PB, by * PB, bz * PB};
-    for (int t = tid; t < PB * PB * PB; t += blockDim.x) {
+    for (int t = tid; t < PB * SX; t += blockDim.x) {
         s_hi[t] = 0;
         s_lo[t] = 0;
     }
     /* the cells that can hold an atom whose spline origin lies in
      * [lo, lo + PW) on every axis: the grid window in the coordinate
      * x + L/2, widened by the distance an atom may have moved since the
-     * cells were filled */
-    int first[3];
+     * cells were filled (and, for FP32 rounding, a little more) */
+    int first[3], num[3];
     for (int d = 0; d < 3; d++) {
-        const float a = (float)lo[d] * pp.h[d] - pp.margin;
+        const float a = (float)lo[d] * pp.h[d] - pp.margin, e = (float)(lo[d] + PW) * pp.h[d] + pp.margin + 0.01f;
         first[d] = pp.ncand[d] >= pp.nc[d] ? 0 : (int)floorf(a / pp.binlen[d]);
+        num[d] = pp.ncand[d] >= pp.nc[d] ? pp.nc[d] : min(pp.ncand[d], (int)floorf(e / pp.binlen[d]) - first[d] + 1);
     }
-    const int nca = pp.ncand[0] * pp.ncand[1] * pp.ncand[2];
-    if (tid < 32) {
-        /* warp 0: ranks and a prefix sum of the candidate cells' atoms */
-        int run = 0;
-        for (int k0 = 0; k0 < nca; k0 += 32) {
-            const int k = k0 + tid;
-            int cnt = 0;
-            if (k < nca) {
-                const int cz = k % pp.ncand[2], cy = (k / pp.ncand[2]) % pp.ncand[1],
-                          cx = k / (pp.ncand[2] * pp.ncand[1]);
-                int c3[3] = {first[0] + cx, first[1] + cy, first[2] + cz};
-                for (int d = 0; d < 3; d++) {
-                    c3[d] %= pp.nc[d];
-                    if (c3[d] < 0) c3[d] += pp.nc[d];
-                }
-                const int r = cell_rank[c3[0] + pp.nc[0] * (c3[1] + pp.nc[1] * c3[2])];
-                const int b = cell_start[r];
-                s_start[k] = b;
-                cnt = cell_start[r + 1] - b;
-            }
-            int incl = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (tid >= o) incl += v;
-            }
-            if (k < nca) s_pre[k] = run + incl - cnt;
-            run += __shfl_sync(0xffffffffu, incl, 31);
+    const int nca = num[0] * num[1] * num[2];
+    for (int k = tid; k < nca; k += blockDim.x) {
+        const int cz = k % num[2], cy = (k / num[2]) % num[1], cx = k / (num[2] * num[1]);
+        int c3[3] = {first[0] + cx, first[1] + cy, first[2] + cz};
+        for (int d = 0; d < 3; d++) {
+            c3[d] %= pp.nc[d];
+            if (c3[d] < 0) c3[d] += pp.nc[d];
         }
-        if (tid == 0) s_pre[nca] = run;
+        const int r = cell_rank[c3[0] + pp.nc[0] * (c3[1] + pp.nc[1] * c3[2])];
+        s_cell[k] = make_int2(cell_start[r], cell_start[r + 1]);
     }
+    if (tid == 0) s_nq = 0;
     __syncthreads();
-    const int total = s_pre[nca];
-    for (int g0 = 0; g0 < total; g0 += blockDim.x) {
-        if (tid == 0) s_nq = 0;
-        __syncthreads();
-        const int g = g0 + tid;
-        if (g < total) {
-            /* the candidate cell: the largest k with s_pre[k] <= g */
-            int lo_k = 0, hi_k = nca;
-            while (hi_k - lo_k > 1) {
-                const int m = (lo_k + hi_k) >> 1;
-                if (s_pre[m] <= g) lo_k = m; else hi_k = m;
-            }
-            const int s = s_start[lo_k] + (g - s_pre[lo_k]);
-            const int4 o = org[s];
-            const float4 a = wq[s];
-            int r[3] = {o.x - lo[0], o.y - lo[1], o.z - lo[2]};
-            bool in = true;
-            for (int d = 0; d < 3; d++) {
-                if (r[d] < 0) r[d] += pp.K[d];
-                in = in && r[d] < PW;
-            }
-            if (in && a.w != 0.0f) {
-                const int slot = atomicAdd(&s_nq, 1);   /* integer sums: the order is free */
-                s_rel[slot] = r[0] | (r[1] << 8) | (r[2] << 16);
-                bspline4(a.x, &s_th[slot][0]);
-                bspline4(a.y, &s_th[slot][4]);
-                bspline4(a.z, &s_th[slot][8]);
-                s_th[slot][12] = a.w;
-            }
-        }
-        __syncthreads();
-        /* one (atom, x point, y point) row of 4 z points per item */
+    /* one (atom, x point, y point) row of 4 z points per item */
+    auto deposit = [&]() {
         const int nw = s_nq * 16;
         for (int t = tid; t < nw; t += blockDim.x) {
             const int at = t >> 4, j = (t >> 2) & 3, k = t & 3;
             const int rl = s_rel[at];
             const int px = (rl & 255) - 3 + j, py = ((rl >> 8) & 255) - 3 + k, pz0 = (rl >> 16) - 3;
             if (px < 0 || px >= PB || py < 0 || py >= PB) continue;
-            const float vxy = s_th[at][12] * s_th[at][j] * s_th[at][4 + k];
-            const int row = (px * PB + py) * PB;
+            const float vxy = s_th[at][j] * s_th[at][4 + k];
+            const float4 tz = *reinterpret_cast<const float4 *>(&s_th[at][8]);
+            const float th[4] = {tz.x, tz.y, tz.z, tz.w};
+            const int row = px * SX + py * SY + pz0;
 #pragma unroll
             for (int l = 0; l < 4; l++) {
-                const int pz = pz0 + l;
-                if (pz < 0 || pz >= PB) continue;
-                const long long iv = __float2ll_rn(vxy * s_th[at][8 + l] * QSCALE);
-                atomicAdd(&s_hi[row + pz], (int)(iv >> 20));
-                atomicAdd(&s_lo[row + pz], (int)(iv & 0xFFFFF));
+                if ((unsigned)(pz0 + l) >= (unsigned)PB) continue;
+                /* hi = rint(v 2^12), lo = rint((v 2^12 - hi) 2^20), by adding
+                 * 1.5 * 2^23 (the integer is then in the low mantissa bits);
+                 * the difference is exact */
+                const float M = 12582912.0f, v = vxy * th[l] * 4096.0f;
+                const float t1 = __fadd_rn(v, M), t2 = __fmaf_rn(__fsub_rn(v, __fsub_rn(t1, M)), 1048576.0f, M);
+                atomicAdd(&s_hi[row + l], __float_as_int(t1) - 0x4B400000);
+                atomicAdd(&s_lo[row + l], __float_as_int(t2) - 0x4B400000);
             }
         }
+    };
+    const int hw = tid >> 4, hl = tid & 15, nhw = blockDim.x >> 4;
+    int k = hw;        /* this half-warp's cell and how far in it is */
+    int off = 0;
+    for (;;) {
+        /* at most 256 atoms a round, so the queue is never overrun */
+        if (k < nca) {
+            const int2 c = s_cell[k];
+            const int s = c.x + off + hl;
+            if (s < c.y) {
+                const int4 o = org[s];
+                const float4 a = wq[s];
+                int r[3] = {o.x - lo[0], o.y - lo[1], o.z - lo[2]};
+                bool in = true;
+                for (int d = 0; d < 3; d++) {
+                    if (r[d] < 0) r[d] += pp.K[d];
+                    in = in && r[d] < PW;
+                }
+                if (in && a.w != 0.0f) {
+                    const int slot = atomicAdd(&s_nq, 1);   /* integer sums: the order is free */
+                    s_rel[slot] = r[0] | (r[1] << 8) | (r[2] << 16);
+                    bspline4(a.x, &s_th[slot][0]);
+                    bspline4(a.y, &s_th[slot][4]);
+                    bspline4(a.z, &s_th[slot][8]);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) s_th[slot][q] *= a.w;
+                }
+            }
+            off += 16;
+            if (c.x + off >= c.y) {
+                k += nhw;
+                off = 0;
+            }
+        }
+        const bool more = __syncthreads_or(k < nca) != 0;
+        if (more && s_nq + 256 <= PQ) {
+            __syncthreads();   /* s_nq is read before the next round adds to it */
+            continue;
+        }
+        deposit();
+        __syncthreads();
+        if (!more) break;
+        if (tid == 0) s_nq = 0;
         __syncthreads();
     }
     for (int t = tid; t < PB * PB * PB; t += blockDim.x) {
         const int px = t / (PB * PB), py = (t / PB) % PB, pz = t % PB;
+        const int at = px * SX + py * SY + pz;
         grid[((size_t)(lo[0] + px) * pp.K[1] + (lo[1] + py)) * pp.K[2] + (lo[2] + pz)] =
-            fmaf((float)s_lo[t], 1.0f / QSCALE, (float)s_hi[t] * (1048576.0f / QSCALE));
+            fmaf((float)s_lo[at], 1.0f / QSCALE, (float)s_hi[at] * (1048576.0f / QSCALE));
     }
 }
 
@@ -251,7 +261,9 @@ __global__ void k_pme_solve(float2 *__restrict__ spec, const float *__restrict__
     }
 }
 
-/* Forces and energies of the reciprocal sum from the convolution grid. */
+/* Forces and energies of the reciprocal sum from the convolution grid, one
+ * thread per atom (four lanes per atom, an x plane each, measured 15 against
+ * 12 us per launch on 64000 ions). */
 template <bool ENERGY>
 __global__ void __launch_bounds__(128) k_pme_gather(pme_par pp, const int4 *__restrict__ org,
                                                     const float4 *__restrict__ wq,
@@ -468,7 +480,13 @@ md_status pme_setup(md_ctx *c, const int K[3])
     }
     c->pme.inv = (int)inv;
     c->pme.plans = 2;
-    if (cufftSetStream(fwd, c->stream) != CUFFT_SUCCESS || cufftSetStream(inv, c->stream) != CUFFT_SUCCESS) {
+    if (cudaStreamCreateWithFlags(&c->pme.stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->pme.fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->pme.join, cudaEventDisableTiming) != cudaSuccess) {
+        pme_free(c);
+        return pme_fail(c, MD_ERR_CUDA, "md_set_pme: stream or event");
+    }
+    if (cufftSetStream(fwd, c->pme.stream) != CUFFT_SUCCESS || cufftSetStream(inv, c->pme.stream) != CUFFT_SUCCESS) {
         pme_free(c);
         return pme_fail(c, MD_ERR_CUDA, "md_set_pme: cufftSetStream failed");
     }
@@ -485,21 +503,37 @@ void pme_free(md_ctx *c)
     cudaFree(c->pme.infl);
     cudaFree(c->pme.org);
     cudaFree(c->pme.wq);
+    if (c->pme.fork) cudaEventDestroy(c->pme.fork);
+    if (c->pme.join) cudaEventDestroy(c->pme.join);
+    if (c->pme.stream) cudaStreamDestroy(c->pme.stream);
     c->pme = md_pme();
 }
 
-void launch_pme(md_ctx *c, const md_kparams &kp, bool energy)
+/* The convolution runs on a stream of its own beside the pair and bonded
+ * kernels, which it shares no data with: it is bound by latency (bricks,
+ * small transforms), they by issue slots.  64000 ions, 112^3 grid, per step:
+ * 161 us in line, 148 beside. */
+void launch_pme_start(md_ctx *c, const md_kparams &kp)
 {
     const pme_par pp = make_pme_par(c);
     const int nbrick = (pp.K[0] / PB) * (pp.K[1] / PB) * (pp.K[2] / PB);
-    k_pme_prep<<<(kp.n + 255) / 256, 256, 0, c->stream>>>(pp, c->x, c->pos4, c->pme.org, c->pme.wq);
-    k_pme_spread<<<nbrick, 256, 0, c->stream>>>(pp, c->pme.org, c->pme.wq, c->cell_rank, c->cell_start,
-                                                c->pme.grid);
+    cudaStream_t s = c->pme.stream;
+    cudaEventRecord(c->pme.fork, c->stream);   /* positions, cells, and the last gather's reads */
+    cudaStreamWaitEvent(s, c->pme.fork, 0);
+    k_pme_prep<<<(kp.n + 255) / 256, 256, 0, s>>>(pp, c->x, c->pos4, c->pme.org, c->pme.wq);
+    k_pme_spread<<<nbrick, 256, 0, s>>>(pp, c->pme.org, c->pme.wq, c->cell_rank, c->cell_start, c->pme.grid);
     cufftExecR2C((cufftHandle)c->pme.fwd, c->pme.grid, (cufftComplex *)c->pme.spec);
     const size_t nspec = (size_t)pp.K[0] * pp.K[1] * (pp.K[2] / 2 + 1);
     const int sb = (int)std::min<size_t>((nspec + 255) / 256, (size_t)c->pme.nsm * 8);
-    k_pme_solve<<<sb, 256, 0, c->stream>>>((float2 *)c->pme.spec, c->pme.infl, nspec);
+    k_pme_solve<<<sb, 256, 0, s>>>((float2 *)c->pme.spec, c->pme.infl, nspec);
     cufftExecC2R((cufftHandle)c->pme.inv, (cufftComplex *)c->pme.spec, c->pme.grid);
+    cudaEventRecord(c->pme.join, s);
+}
+
+void launch_pme_finish(md_ctx *c, const md_kparams &kp, bool energy)
+{
+    const pme_par pp = make_pme_par(c);
+    cudaStreamWaitEvent(c->stream, c->pme.join, 0);
     const int nb = (kp.n + 127) / 128;
     if (energy)
         k_pme_gather<true><<<nb, 128, 0, c->stream>>>(pp, c->pme.org, c->pme.wq, c->pme.grid, c->f, c->epot);

@@ -181,6 +181,8 @@ struct md_pme {
     float4 *wq = nullptr;          /* per sorted atom: offsets (x, y, z) and charge */
     int fwd = 0, inv = 0;          /* cuFFT plans (cufftHandle) */
     int plans = 0;                 /* plans created */
+    cudaStream_t stream = nullptr; /* the convolution's, beside the pair kernel's */
+    cudaEvent_t fork = nullptr, join = nullptr;
     int excl = 0;                  /* the system has excluded pairs to remove */
     int nsm = 1;
     float e_bg = 0.0f;             /* background energy of a net charge, per atom */
@@ -345,8 +347,11 @@ inline void md_shift_consts(int lkspace, float rcutsq, float alfa, float reacf, 
 /* grid K (all zero: off); lkspace 2 single systems only (md_set_pme checks) */
 md_status pme_setup(md_ctx *c, const int K[3]);
 void pme_free(md_ctx *c);
-/* spread, FFTs, solve and gather of the reciprocal sum, added into the forces */
-void launch_pme(md_ctx *c, const md_kparams &kp, bool energy);
+/* the reciprocal sum: spread, FFTs and solve on the context's second stream
+ * from the positions as they are, then, back on c->stream, the gather into
+ * the forces */
+void launch_pme_start(md_ctx *c, const md_kparams &kp);
+void launch_pme_finish(md_ctx *c, const md_kparams &kp, bool energy);
 /* Waits for the copies from pageable memory and the memsets issued so far:
  * they run on the legacy default stream and may still be under way when the
  * call returns, and a context's own stream (non-blocking) does not wait for
