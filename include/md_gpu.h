@@ -282,8 +282,12 @@ md_status md_set_tuning(md_ctx *ctx, int pair_tpa, int list_tpa);
 /* List entries each pair-kernel lane loads per batch (memory-level
  * parallelism against registers): 0 = the default for the lane count (8 for
  * 1-4 lanes, 4 for 8, 2 for 16, 1 for 32); also half the default at 4, 8
- * and 16 lanes.  A new context has 8 lanes and 2 entries; md_set_tuning
- * resets the entries to 0. */
+ * and 16 lanes.  A new context has 8 lanes and 2 entries, or by its size, a
+ * single system of few atoms, 32 or 16 lanes and their default (up to one
+ * block of 8 atoms, two of 16 per SM: 1208 and 4848 atoms on 152 SMs; 16 at
+ * most with the reciprocal sum);
+ * a depth set before any other tuning brings such a context to 8 lanes.
+ * md_set_tuning resets the entries to 0. */
 md_status md_set_pair_depth(md_ctx *ctx, int depth);
 /* Autotuner: times the pair kernel for 2/4/8/16 threads per atom (also at
  * 4/8/16 threads with half the default entries per lane and batch) and the

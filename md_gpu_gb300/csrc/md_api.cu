@@ -549,6 +549,33 @@ struct host_stage {
     }
 };
 
+/* Lanes per atom of a new single system, by its size: the most with which the
+ * run of steps in one launch (k_run.cu: blocks of 256 / lanes atoms and one
+ * more) has one block per SM at 32 lanes or two at 16, else 8.  A small
+ * system's step is a chain of latencies, and more lanes shorten the part of
+ * it that walks a row.  us per step at 8 / 16 / 32 lanes: 500 LJ atoms 7.1 /
+ * 6.4 / 6.3, 982 ions 12.0 / 9.5 / 9.0, 1536 water atoms 18.5 / 14.4 / 15.4,
+ * 2048 LJ atoms 7.6 / 6.5 / 7.5, 4080 ions 12.9 / 11.6 / 26 (too many
+ * blocks), 8000 ions 16.2 / 28.4 / - .  With the reciprocal sum, whose kernels
+ * run beside the pair kernel, 16 at most: 1000 ions 45.5 / 45.0 / 49.0, 2744
+ * ions 51.6 / 48.2 / 50.6.  Picked after the first forces, which 8 lanes
+ * computed: a context then brought to 8 lanes runs as if it had had them all
+ * along. */
+static void pick_lanes(md_ctx *c)
+{
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    const int lanes = (c->n + 7) / 8 + 1 <= nsm && !c->pme.on ? 32 : (c->n + 15) / 16 + 1 <= 2 * nsm ? 16 : 8;
+    if (lanes == 8) return;
+    c->pair_tpa = lanes;
+    c->pair_depth = 0;
+    c->lanes_by_size = 1;
+}
+
 /* Streams, device memory, upload, first list build and force evaluation of
  * a context whose host fields are set; frees everything on failure. */
 md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
@@ -682,6 +709,7 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
     if (s == MD_OK) s = initial_build(c);
     if (s == MD_OK) s = refresh_state(c);
     if (s == MD_OK) default_step_form(c);
+    if (s == MD_OK && !c->batch) pick_lanes(c);
     if (s != MD_OK) {
         g_last_error = c->last_error;
         md_destroy(c);
@@ -2235,6 +2263,7 @@ md_status md_set_pme(md_ctx *c, int k0, int k1, int k2)
     md_status s = pme_setup(c, K);
     if (s != MD_OK) return s;
     default_step_form(c);
+    if (c->lanes_by_size) pick_lanes(c);
     return refresh_state(c);   /* the forces (and record) of the current state with the new sum */
 }
 
@@ -2252,6 +2281,7 @@ md_status md_autotune(md_ctx *c, int *pair_tpa, int *list_tpa)
 {
     if (!c) return MD_ERR_ARG;
     c->form_chosen = 1;
+    c->lanes_by_size = 0;
     const int lt[] = {0, 4, 8, 16};
     float best = 1e30f;
     int bp = c->pair_tpa, bl = c->list_tpa, bf = 0;
@@ -2494,11 +2524,14 @@ md_status md_set_fused_step(md_ctx *c, int fused)
 md_status md_set_pair_depth(md_ctx *c, int depth)
 {
     if (!c) return MD_ERR_ARG;
-    const int t = c->pair_tpa;
+    /* lanes picked by size at creation give way to the 8 that depths are for */
+    const int t = c->lanes_by_size ? 8 : c->pair_tpa;
     const int def = t >= 32 ? 1 : (t >= 16 ? 2 : (t >= 8 ? 4 : 8));
     if (depth == def) depth = 0;
     const bool ok = depth == 0 || (t == 4 && depth == 4) || (t == 8 && depth == 2) || (t == 16 && depth == 1);
     if (!ok) return fail(c, MD_ERR_ARG, "md_set_pair_depth: depth not built for this lane count");
+    c->pair_tpa = t;
+    c->lanes_by_size = 0;
     c->pair_depth = depth;
     if (c->gexec) {
         cudaGraphExecDestroy(c->gexec);
@@ -2515,6 +2548,7 @@ md_status md_set_tuning(md_ctx *c, int pair_tpa, int list_tpa)
     if (c->batch && list_tpa != 0)
         return fail(c, MD_ERR_ARG, "md_set_tuning: a batch builds its lists one warp per cell");
     c->pair_tpa = pair_tpa;
+    c->lanes_by_size = 0;
     c->pair_depth = 0;
     c->list_tpa = list_tpa;
     if (c->gexec) {

@@ -270,10 +270,11 @@ struct md_ctx {
     double *io_dev = nullptr;      /* 4*pitch doubles for host transfers */
     int pair_tpa = 8;    /* threads per atom in the pair kernel */
     /* list entries per lane and batch (0: the default for pair_tpa).  A new
-     * context takes two at its 8 lanes: fewer registers, more warps (against
+     * context of 8 lanes takes two: fewer registers, more warps (against
      * four: 64000 ions 43 against 47 us, 98304 water atoms 119 against 143
      * us, 128 replicas of 512 to 8000 ions 259 against 340 us per launch) */
     int pair_depth = 2;
+    int lanes_by_size = 0;   /* 1: pair_tpa was picked at creation (pick_lanes) and nothing chosen since */
     int centered = 0;    /* every position in [-L/2, L/2] (set at upload; the wraps keep it) */
     int list_tpa = 0;    /* list build: 0 = one warp per cell, else threads per atom */
     int fp64 = 0;        /* 1: force kernels in FP64 on the FP64 positions (md_set_precision) */

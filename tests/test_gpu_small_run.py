@@ -80,3 +80,34 @@ def test_list_after_creation():
             counts.append(sim.neighbor_list(128)[1])
     assert counts[0][:1372].min() > 0
     assert all(np.array_equal(c, counts[0]) for c in counts)
+
+
+@pytest.mark.parametrize("natom,lanes", [(510, 32), (1208, 32), (1210, 16), (4848, 16), (4850, 8)])
+def test_lanes_by_size(natom, lanes):
+    """A new single system's lanes per atom follow its size (152 SMs: 1208 and
+    4848 atoms are the last of 32 and 16 lanes).  The forces differ from those
+    of 8 lanes by the rounding of FP32 sums only: both are within 1e-5 (rms,
+    relative) of the FP64 forces, hence within 2e-5 of each other.  A depth
+    set first brings the context to the 8 lanes that it was built for."""
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("sizes are for 152 SMs")
+    arrays = synth.to_arrays(synth.nacl_replica(seed=6, natom=natom, integrator="leapfrog"))
+    F = []
+    for first in (lambda s: None, lambda s: s.set_tuning(8, 0), lambda s: s.set_tuning(8, 0, 2)):
+        with MDSystem.from_arrays(**arrays) as sim:
+            assert sim.info()["pair_tpa"] == lanes
+            first(sim)
+            sim.compute_forces()
+            F.append(sim.forces()[:, :3])
+            sim.step(5)
+            F.append(sim.forces()[:, :3])
+    for k in (0, 1):
+        d = np.sqrt(((F[k] - F[2 + k]) ** 2).mean() / (F[2 + k] ** 2).mean())
+        assert d <= 2e-5
+        assert np.array_equal(F[2 + k], F[4 + k])
+    with MDSystem.from_arrays(**arrays) as sim:
+        from md_gpu_gb300.system import library
+        for depth, ok in ((1, False), (4, True), (2, True)):
+            assert (library().md_set_pair_depth(sim._ctx, depth) == 0) == ok
+        assert sim.info()["pair_tpa"] == 8 and sim.info()["pair_depth"] == 2
