@@ -58,14 +58,15 @@ __global__ void __launch_bounds__(128, B > 2 ? 1 : ENERGY || KIND == 1 ? 8 : 7) 
     }
 }
 
-/* The end of an integrator block of replica rep: as block_close, with the
- * sums going to the replica's accumulators and a moved atom raising the
- * replica's rebuild request too.  Returns true in every thread of the last
- * block to finish.  Thread 0 alone fences: the other threads' stores are
- * read by later kernels only. */
-__device__ __forceinline__ bool block_close_b(long long a, long long b, long long c, int nsum, bool moved, int rep,
-                                              unsigned long long *racc, int *rep_upd, md_devstate *st,
-                                              unsigned *counter, long long *sh)
+/* The end of an integrator block: as block_close, with the sums (nsum > 0)
+ * going to the accumulators acc and a moved atom raising the replica's rebuild
+ * request *upd too; the block is counted in *counter.  Returns true in every
+ * thread of the block that is the last of `blocks`.  Thread 0 alone fences:
+ * the other threads' stores are read by later kernels only. */
+template <class CNT>
+__device__ __forceinline__ bool block_close_b(long long a, long long b, long long c, int nsum, bool moved, int *upd,
+                                              unsigned long long *acc, md_devstate *st, CNT *counter, CNT blocks,
+                                              long long *sh)
 {
     __shared__ bool last;
     if (nsum > 0) {
@@ -93,102 +94,117 @@ __device__ __forceinline__ bool block_close_b(long long a, long long b, long lon
                 tb += sh[nw + k];
                 tc += sh[2 * nw + k];
             }
-            atomicAdd(racc + 3 * rep, (unsigned long long)ta);
+            atomicAdd(acc, (unsigned long long)ta);
             if (nsum > 1) {
-                atomicAdd(racc + 3 * rep + 1, (unsigned long long)tb);
-                atomicAdd(racc + 3 * rep + 2, (unsigned long long)tc);
+                atomicAdd(acc + 1, (unsigned long long)tb);
+                atomicAdd(acc + 2, (unsigned long long)tc);
             }
         }
         if (any) {
             st->update = 1;
-            rep_upd[rep] = 1;
+            *upd = 1;
         }
         __threadfence();
-        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        last = atomicAdd(counter, (CNT)1) == blocks - 1;
         __threadfence();
     }
     __syncthreads();
     return last;
 }
 
-/* Four sums over the block at once (each as block_sum); valid in thread 0. */
-__device__ __forceinline__ void block_sum4(double (&v)[4], double (*sh)[4])
+/* Four sums over the first `count` threads of the block at once, the others'
+ * terms being zero (each in the order of a whole block's shuffle tree); valid
+ * in thread 0.  Called by every thread of the block. */
+__device__ __forceinline__ void block_sum4(double (&v)[4], double (*sh)[4], int count)
 {
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int q = 0; q < 4; q++) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0)
+    const int nw = min((count + 31) >> 5, (int)(blockDim.x >> 5));
+    if (w < nw) {
+        for (int o = 16; o > 0; o >>= 1) {
+            if (o >= count) continue;   /* adds zeros only */
 #pragma unroll
-        for (int q = 0; q < 4; q++) sh[w][q] = v[q];
+            for (int q = 0; q < 4; q++) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+        }
+        if (l == 0)
+#pragma unroll
+            for (int q = 0; q < 4; q++) sh[w][q] = v[q];
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < 4; q++) v[q] = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++)
+        for (int k = 0; k < nw; k++)
 #pragma unroll
             for (int q = 0; q < 4; q++) v[q] += sh[k][q];
     }
 }
 
-/* NPT: after a leapfrog step, the replica's box scaled by the factor the
- * step applied to its positions, and what the kernels derive from it: the
- * FP32 box and its inverse as the reference rounds it (simulation.cu:
- * 290-292), 2/L, the wrap limit and the cell side.  The cell grid keeps its
- * cell counts and stencil until the host lays it out again (md_step does
- * between chunks of at most 128 steps, before the grid's 3% margin can be
- * used up at the per-step clamp of mu, 1e-4), so a box whose cells shrink
- * below half the list radius inside a chunk, or whose list radius exceeds
- * half the box, can no longer be listed correctly: that sets the sticky
- * status 2, which the host reports.  Runs in the last block of the step's
- * leapfrog, when no other block reads the table any more. */
-__device__ void npt_box(md_rep &R, double mu, md_devstate *st)
+/* NPT: after a leapfrog step, axis d of the replica's box (L before it)
+ * scaled by the factor the step applied to its positions, and what the
+ * kernels derive from it: the FP32 box and its inverse as the reference
+ * rounds it (simulation.cu:290-292), 2/L (twice 1/L, which rounds alike), the
+ * wrap limit and the cell side.  The cell grid keeps its cell counts and
+ * stencil until the host lays it out again (md_step does between chunks of
+ * at most 128 steps, before the grid's 3% margin can be used up at the
+ * per-step clamp of mu, 1e-4), so a box whose cells shrink below half the
+ * list radius inside a chunk, or whose list radius exceeds half the box, can
+ * no longer be listed correctly: that sets the sticky status 2, which the
+ * host reports.  Runs in the last block of the replica's leapfrog, when no
+ * other block reads its table entry any more. */
+__device__ void npt_box_axis(md_rep &R, int d, double L0, double mu, md_devstate *st)
 {
-    bool bad = false;
-    for (int d = 0; d < 3; d++) {
-        const double L = R.boxd[d] * mu;
-        R.boxd[d] = L;
-        R.box[d] = (float)L;
-        R.boxi[d] = (float)(1.0 / L);
-        R.box2i[d] = 2.0 / L;
-        R.wlim[d] = 0.4999f * R.box[d];
-        R.binlen[d] = R.box[d] / (float)R.ncell[d];
-        if (R.stencil[d] >= 0 && R.binlen[d] < R.rl_half) bad = true;
-        if (2.0f * R.rl_half > 0.5f * R.box[d]) bad = true;
-    }
-    if (bad) atomicOr(&st->status, 2);
+    const double L = L0 * mu, inv = 1.0 / L;
+    const float box = (float)L, binlen = box / (float)R.ncell[d];
+    R.boxd[d] = L;
+    R.box[d] = box;
+    R.boxi[d] = (float)inv;
+    R.box2i[d] = 2.0 * inv;
+    R.wlim[d] = 0.4999f * box;
+    R.binlen[d] = binlen;
+    if ((R.stencil[d] >= 0 && binlen < R.rl_half) || 2.0f * R.rl_half > 0.5f * box) atomicOr(&st->status, 2);
 }
 
-/* Runs in the last block to finish: one thread per replica turns its
- * accumulators into KE, PE and virial (and clears them for the next step),
- * then does the replica's thermostat bookkeeping; the batch's step record
- * sums the replicas in a fixed order. */
-__device__ void finalize_b(const md_kparams &kp, const thermo_par &tp, int mode, int nrep,
-                           md_rep *reps, md_repstate *repst, unsigned long long *racc, md_devstate *st,
-                           md_thermo *rec, int rec_cap, double *rep_hist, double (*sh)[4])
+/* The end of a step for replica r, by the last of its blocks: thread 0 turns
+ * the accumulators into KE, PE and virial (and clears them) and does the
+ * replica's thermostat bookkeeping, a second warp the pressure and a third
+ * the box (NPT).  FP64 arithmetic on a few values is a chain of latencies on
+ * this GPU's narrow FP64 pipe: with every replica in the last block of the
+ * batch this end took 24 us of a step of 128 replicas and 12 us of a single
+ * NPT replica (one thread each); here replicas overlap with each other and
+ * with the blocks still running: 482 -> 473 us per step of 128 replicas of
+ * 512 to 8000 ions, 463 -> 457 of 512 replicas, 33.9 -> 28.0 of one NPT
+ * system of 7986 ions.  The last replica to come then sums the batch's step
+ * record over the replicas in a fixed order.  racc: 3 sums per replica, then
+ * its count of finished blocks, then its 4 terms of the record.  Returns true
+ * in thread 0 of the batch's last block. */
+__device__ bool finalize_b(const md_kparams &kp, const thermo_par &tp, int mode, int nrep, int r, md_rep *reps,
+                           md_repstate *repst, unsigned long long *racc, const step_io &io, double (*sh)[4])
 {
-    double tke = 0.0, tpe = 0.0, tw = 0.0, tex = 0.0;
-    /* the step this record belongs to (thread 0 advances it after the sums) */
+    __shared__ bool all;
+    const int wp = threadIdx.x >> 5, l = threadIdx.x & 31;
+    md_devstate *st = io.st;
+    md_rep &R = reps[r];
+    md_repstate &S = repst[r];
+    volatile unsigned long long *acc = racc + 3 * r;
+    double *rtot = reinterpret_cast<double *>(racc + 4 * nrep);
+    const bool npt = tp.npt && mode == 0;
+    /* the step this record belongs to (the batch's last block advances it) */
     const long long step = ((volatile md_devstate *)st)->step;
     const int builds = ((volatile md_devstate *)st)->builds;
-    double *hist = (rep_hist && mode != 2) ? rep_hist + (size_t)(step & (rec_cap - 1)) * 3 * nrep : nullptr;
-    for (int r = threadIdx.x; r < nrep; r += blockDim.x) {
-        md_rep &R = reps[r];
-        const double a = fix_take(racc + 3 * r, MD_KFIX);
-        double b = fix_take(racc + 3 * r + 1, MD_EFIX);
-        double c = fix_take(racc + 3 * r + 2, MD_EFIX);
-        if (tp.npt && mode == 0) {
-            /* P = (2 KE + sum_pairs F.r) / (3 V); c = sum over atoms of ff r^2,
-             * every pair counted from both atoms; V of the box the forces saw */
-            const double V = R.boxd[0] * R.boxd[1] * R.boxd[2];
-            const double P = (2.0 * a + 0.5 * c) / (3.0 * V);
-            double mu = 1.0 - R.mu_k * (R.p0 - P);
-            mu = fmin(fmax(mu, 1.0 - R.mu_max), 1.0 + R.mu_max);
-            repst[r].pressure = P;
-            repst[r].mu_used = repst[r].mu_next;
-            repst[r].mu_next = mu;
-            if (R.npt) npt_box(R, repst[r].mu_used, st);
-        }
+    double a = 0.0, b = 0.0, c = 0.0, L0 = 0.0, V = 0.0, mu0 = 1.0;
+    if (l == 0 && wp < 2) {
+        a = (double)(long long)acc[0] / MD_KFIX;
+        b = (double)(long long)acc[1] / MD_EFIX;
+        c = (double)(long long)acc[2] / MD_EFIX;
+    }
+    if (npt && wp == 1) V = R.boxd[0] * R.boxd[1] * R.boxd[2];
+    if (npt && wp == 2 && l < 3) L0 = R.boxd[l];
+    if (npt) mu0 = S.mu_next;
+    __syncthreads();   /* read above, written below */
+    double tot[4] = {0.0, 0.0, 0.0, 0.0};
+    if (threadIdx.x == 0) {
+        acc[0] = acc[1] = acc[2] = 0ull;
+        racc[3 * nrep + r] = 0ull;
         if (!tp.energy) b = c = 0.0;
         thermo_par t = tp;
         t.t0 = R.t0;
@@ -197,30 +213,58 @@ __device__ void finalize_b(const md_kparams &kp, const thermo_par &tp, int mode,
         t.inv_ndfr = R.inv_ndfr;
         t.inv_q = R.inv_q;
         double xi, eta, lam;
-        double ke = thermo_advance(kp.dt, t, mode, a, b, c, repst + r, &xi, &eta, &lam);
-        tke += ke;
-        tpe += b;
-        tw += c;
+        const double ke = thermo_advance(kp.dt, t, mode, a, b, c, &S, &xi, &eta, &lam);
         const double ex = t.nh ? 0.5 * t.q_nh * xi * xi + t.ndf * RGAS * t.t0 * eta : 0.0;
-        tex += ex;
-        if (hist) {
-            hist[3 * r] = ke;
-            hist[3 * r + 1] = tp.energy ? b : 0.0;
-            hist[3 * r + 2] = tp.energy ? ke + b + ex : 0.0;
+        tot[0] = ke;
+        tot[1] = b;
+        tot[2] = c;
+        tot[3] = ex;
+        if (nrep > 1)
+            for (int q = 0; q < 4; q++) rtot[4 * r + q] = tot[q];
+        if (io.rep_hist && mode != 2) {
+            double *hist = io.rep_hist + ((size_t)(step & (io.rec_cap - 1)) * nrep + r) * 3;
+            hist[0] = ke;
+            hist[1] = tp.energy ? b : 0.0;
+            hist[2] = tp.energy ? ke + b + ex : 0.0;
         }
+    } else if (npt && wp == 1 && l == 0) {
+        /* P = (2 KE + sum_pairs F.r) / (3 V); c = sum over atoms of ff r^2,
+         * every pair counted from both atoms; V of the box the forces saw */
+        const double P = (2.0 * a + 0.5 * c) / (3.0 * V);
+        double mu = 1.0 - R.mu_k * (R.p0 - P);
+        mu = fmin(fmax(mu, 1.0 - R.mu_max), 1.0 + R.mu_max);
+        S.pressure = P;
+        S.mu_used = mu0;
+        S.mu_next = mu;
+    } else if (npt && R.npt && wp == 2 && l < 3) {
+        npt_box_axis(R, l, L0, mu0, st);
     }
-    double tot[4] = {tke, tpe, tw, tex};
-    block_sum4(tot, sh);
-    if (threadIdx.x != 0) return;
+    if (nrep > 1) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            all = atomicAdd(io.counter, 1u) == (unsigned)nrep - 1u;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!all) return false;
+        for (int q = 0; q < 4; q++) tot[q] = 0.0;
+        for (int k = threadIdx.x; k < nrep; k += blockDim.x)
+            for (int q = 0; q < 4; q++) tot[q] += __ldcg(rtot + 4 * k + q);
+        block_sum4(tot, sh, nrep);
+    }
+    if (threadIdx.x != 0) return false;
     const double KE = tot[0], PE = tot[1], W = tot[2], EX = tot[3];
+    *io.counter = 0;
     st->ke = KE;
     if (tp.energy) {
         st->pe = PE;
         st->virial = W / 6.0;
     }
-    if (mode == 2) return;
+    if (mode == 2) return true;
     st->temper = 2.0 * KE * tp.inv_ndfr;
-    write_record(tp, tp.inv_ndfr, KE, PE, W, EX, 0.0, 1.0, step, builds, st, rec, rec_cap);
+    write_record(tp, tp.inv_ndfr, KE, PE, W, EX, 0.0, 1.0, step, builds, st, io.rec, io.rec_cap);
+    return true;
 }
 
 /* Leapfrog of a batch (k_leapfrog per replica, one thread per (atom, axis)):
@@ -278,13 +322,10 @@ __global__ void __launch_bounds__(3 * MD_LA) k_leapfrog_b(md_kparams kp, thermo_
         pos4[s] = p;
         moved = md_rsq_box(p, io.pos_old[s], R.box, R.boxi) >= R.rmaxdif;
     }
-    if (block_close_b(ke, pe, w, tp.energy || tp.npt ? 3 : 1, moved, bt.x, racc, rep_upd, io.st, io.counter, shl)) {
-        finalize_b(kp, tp, 0, nrep, reps, repst, racc, io.st, io.rec, io.rec_cap, io.rep_hist, sh);
-        if (threadIdx.x == 0) {
-            set_condition(io);
-            *io.counter = 0;
-        }
-    }
+    if (block_close_b(ke, pe, w, tp.energy || tp.npt ? 3 : 1, moved, rep_upd + bt.x, racc + 3 * bt.x, io.st,
+                      racc + 3 * nrep + bt.x, (unsigned long long)R.nblk, shl) &&
+        finalize_b(kp, tp, 0, nrep, bt.x, reps, repst, racc, io, sh))
+        set_condition(io);
 }
 
 /* Velocity Verlet first half of a batch (k_vv_first per replica). */
@@ -329,7 +370,8 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_first_b(md_kparams kp, step_io
         }
         return;
     }
-    if (block_close_b(0, 0, 0, 0, moved, bt.x, nullptr, rep_upd, io.st, io.counter, nullptr) && threadIdx.x == 0) {
+    if (block_close_b(0, 0, 0, 0, moved, rep_upd + bt.x, nullptr, io.st, io.counter, gridDim.x, nullptr) &&
+        threadIdx.x == 0) {
         set_condition(io);
         *io.counter = 0;
     }
@@ -371,10 +413,9 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_second_b(md_kparams kp, thermo
             w = llrint((double)vir[s] * MD_EFIX);
         }
     }
-    if (block_close_b(ke, pe, w, tp.energy ? 3 : 1, false, bt.x, racc, nullptr, io.st, io.counter, shl)) {
-        finalize_b(kp, tp, do_kick ? 1 : 2, nrep, reps, repst, racc, io.st, io.rec, io.rec_cap, io.rep_hist, sh);
-        if (threadIdx.x == 0) *io.counter = 0;
-    }
+    if (block_close_b(ke, pe, w, tp.energy ? 3 : 1, false, nullptr, racc + 3 * bt.x, io.st, racc + 3 * nrep + bt.x,
+                      (unsigned long long)R.nblk, shl))
+        finalize_b(kp, tp, do_kick ? 1 : 2, nrep, bt.x, reps, repst, racc, io, sh);
 }
 
 template <int KIND, bool ENERGY>

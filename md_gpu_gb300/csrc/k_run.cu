@@ -28,7 +28,7 @@
  * update -> barrier of one step, and the rebuilds.  Whole md_step calls of
  * 100 steps against the step graphs: 500 LJ atoms 2.48 -> 0.75 ms, 4000 LJ
  * atoms 2.71 -> 1.00 ms, 982 ions 3.30 -> 1.01 ms; 20 steps of 5184 water
- * atoms 1.58 -> 0.74 ms (rebuilds in every second step).  Above the resident
+ * atoms 1.58 -> 0.74 ms.  Above the resident
  * blocks the step graphs are the only form (8000 ions: 16.2 us per step here,
  * 28.4 with 16 lanes per atom, where they do not fit).  Copying the block's
  * list rows to shared memory at each rebuild was no faster (12.8 against

@@ -624,7 +624,7 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
     if (batch) {
         MD_ALLOC(c->reps_dev, c->nrep); MD_ALLOC(c->repst, c->nrep);
         MD_ALLOC(c->arep, P); MD_ALLOC(c->crep, c->ncells);
-        MD_ALLOC(c->rep_upd, c->nrep); MD_ALLOC(c->racc, 3 * (size_t)c->nrep);
+        MD_ALLOC(c->rep_upd, c->nrep); MD_ALLOC(c->racc, 8 * (size_t)c->nrep);
         MD_ALLOC(c->ljr_dev, (size_t)MD_MAXTYPE * MD_MAXTYPE * c->nrep);
         MD_ALLOC(c->grid_tab, h.grid.size());
         MD_ALLOC(c->rep_hist, (size_t)c->rec_cap * 3 * c->nrep);
@@ -691,7 +691,7 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
         up(c->ljr_dev, h.ljr.data(), sizeof(float2) * h.ljr.size());
         up(c->grid_tab, h.grid.data(), sizeof(int2) * h.grid.size());
         if (e == cudaSuccess) e = cudaMemset(c->rep_upd, 0, sizeof(int) * c->nrep);
-        if (e == cudaSuccess) e = cudaMemset(c->racc, 0, sizeof(unsigned long long) * 3 * c->nrep);
+        if (e == cudaSuccess) e = cudaMemset(c->racc, 0, sizeof(unsigned long long) * 8 * c->nrep);
     }
     if (e == cudaSuccess) e = cudaMemset(c->f, 0, sizeof(long long) * 3 * P);
     if (e == cudaSuccess) e = cudaMemset(c->vir, 0, sizeof(float) * P);
@@ -1656,7 +1656,7 @@ static std::vector<snap_part> snap_parts(md_ctx *c)
         {c->vir, P * sizeof(float)},        {c->epot, P * sizeof(float)}};
     if (c->batch) {
         v.push_back({c->repst, c->nrep * sizeof(md_repstate)});
-        v.push_back({c->racc, 3 * (size_t)c->nrep * sizeof(unsigned long long)});
+        v.push_back({c->racc, 8 * (size_t)c->nrep * sizeof(unsigned long long)});
         v.push_back({c->rep_upd, c->nrep * sizeof(int)});
         v.push_back({c->reps_dev, c->nrep * sizeof(md_rep)});   /* NPT moves the boxes */
     }

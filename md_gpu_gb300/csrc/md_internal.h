@@ -293,7 +293,9 @@ struct md_ctx {
     int *rep_upd = nullptr;       /* per replica: an atom moved >= skin/2 since its last build */
     int *crep = nullptr;          /* cell rank -> replica */
     float2 *ljr_dev = nullptr;    /* nrep x 64 (lj1, lj2) */
-    unsigned long long *racc = nullptr; /* nrep x 3 fixed-point KE, PE, virial sums of a step */
+    /* nrep x 3 fixed-point KE, PE, virial sums of a step, nrep counts of
+     * finished integrator blocks, nrep x 4 FP64 terms of the step record */
+    unsigned long long *racc = nullptr;
     int2 *grid_tab = nullptr;     /* the MD_NGRID replica-aligned grids, concatenated */
     int grid_off[MD_NGRID] = {0}, grid_cnt[MD_NGRID] = {0};
 
