@@ -111,3 +111,20 @@ def test_lanes_by_size(natom, lanes):
         for depth, ok in ((1, False), (4, True), (2, True)):
             assert (library().md_set_pair_depth(sim._ctx, depth) == 0) == ok
         assert sim.info()["pair_tpa"] == 8 and sim.info()["pair_depth"] == 2
+
+
+def test_large_forces_match_separate_kernels():
+    """Two atoms 0.45 sigma apart: forces above 2^18 take the run's
+    general force conversion and still give the separate kernels' bits."""
+    a = synth.to_arrays(synth.argon_fcc(ncell=5, seed=3, integrator="vv"))
+    a["pos"] = np.array(a["pos"], copy=True)
+    a["pos"][1] = a["pos"][0] + np.array([0.45, 0.0, 0.0], a["pos"].dtype)
+    out = []
+    for graphs in (True, False):
+        with MDSystem.from_arrays(**a) as sim:
+            sim.set_graphs(graphs)
+            assert np.abs(sim.forces()[:2, 0]).min() > 2.0 ** 18
+            sim.step(4)
+            out.append((sim.positions(), sim.velocities(), sim.forces()))
+    for p, q in zip(*out):
+        assert np.array_equal(p, q)
