@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_first_b(md_kparams kp, step_io
 
 /* Velocity Verlet second half of a batch (k_vv_second per replica); do_kick
  * = 0 observes the state only. */
-__global__ void __launch_bounds__(3 * MD_LA) k_vv_second_b(md_kparams kp, thermo_par tp,
+__global__ void __launch_bounds__(3 * MD_LA, 4) k_vv_second_b(md_kparams kp, thermo_par tp,
                                                           int do_kick, step_io io, int nrep,
                                                           const int2 *__restrict__ tab,
                                                           md_rep *reps, md_repstate *repst,
@@ -418,6 +418,56 @@ __global__ void __launch_bounds__(3 * MD_LA) k_vv_second_b(md_kparams kp, thermo
     if (block_close_b(ke, pe, w, tp.energy ? 3 : 1, false, nullptr, racc + 3 * bt.x, io.st, racc + 3 * nrep + bt.x,
                       (unsigned long long)R.nblk, shl))
         finalize_b(kp, tp, do_kick ? 1 : 2, nrep, bt.x, reps, repst, racc, io, sh);
+}
+
+/* k_vv_second_b and the next step's k_vv_first_b as one kernel (k_vv_mid per
+ * replica). */
+__global__ void __launch_bounds__(3 * MD_LA, 4) k_vv_mid_b(md_kparams kp, thermo_par tp, step_io io, int nrep,
+                                                          const int2 *__restrict__ tab, md_rep *reps,
+                                                          md_repstate *repst, int *rep_upd,
+                                                          unsigned long long *racc, double *x, double *v,
+                                                          const double *__restrict__ mass,
+                                                          const double *__restrict__ kick, float4 *pos4,
+                                                          const long long *__restrict__ f,
+                                                          const float *__restrict__ epot,
+                                                          const float *__restrict__ vir)
+{
+    __shared__ double sh[3 * MD_LA / 32][4];
+    __shared__ long long shl[3 * (3 * MD_LA / 32)];
+    __shared__ float s_x[3][MD_LA];
+    pdl_wait();   /* the forces of this step */
+    const int2 bt = tab[blockIdx.x];
+    const md_rep &R = reps[bt.x];
+    const int d = threadIdx.x / MD_LA, a = threadIdx.x - d * MD_LA;
+    const int s = bt.y + a;
+    const bool act = s < R.atom0 + R.natom;
+    const size_t o = (size_t)d * kp.pitch + s;
+    long long ke = 0, pe = 0, w = 0;
+    if (act) {
+        const axis_par ax = axis_of(d, R.wlim, R.boxd, R.box2i);
+        const double fd = (double)f[o], hk = 0.5 * kick[s];
+        double vv = fma(fd, hk, v[o]);
+        ke = ke_fix(mass[s], vv);
+        vv = fma(fd, hk, vv);
+        v[o] = vv;
+        double xx = x[o] + vv * kp.dt;
+        s_x[d][a] = wrap(xx, ax.lim, ax.L, ax.two_over_l);
+        x[o] = xx;
+        if (d == 0 && tp.energy) {
+            pe = llrint((double)epot[s] * MD_EFIX);
+            w = llrint((double)vir[s] * MD_EFIX);
+        }
+    }
+    __syncthreads();
+    bool moved = false;
+    if (d == 0 && act) {
+        float4 p = make_float4(s_x[0][a], s_x[1][a], s_x[2][a], pos4[s].w);
+        pos4[s] = p;
+        moved = md_rsq_box(p, io.pos_old[s], R.box, R.boxi) >= R.rmaxdif;
+    }
+    if (block_close_b(ke, pe, w, tp.energy ? 3 : 1, moved, rep_upd + bt.x, racc + 3 * bt.x, io.st,
+                      racc + 3 * nrep + bt.x, (unsigned long long)R.nblk, shl))
+        finalize_b(kp, tp, 1, nrep, bt.x, reps, repst, racc, io, sh);
 }
 
 template <int KIND, bool ENERGY>
@@ -489,6 +539,14 @@ void launch_vv_first_b(md_ctx *c, const md_kparams &kp, unsigned long long cond,
                                                            grid_int(c), c->reps_dev, c->repst,
                                                            c->rep_upd, c->x, c->v, c->kick, c->pos4,
                                                            c->f);
+}
+
+void launch_vv_mid_b(md_ctx *c, const md_kparams &kp, int energy)
+{
+    md_launch_pdl(k_vv_mid_b, dim3(grid_int_blocks(c)), dim3(3 * MD_LA), c->stream, kp, make_tp(c, energy),
+                  make_io(c, 0, 0), c->nrep, grid_int(c), c->reps_dev, c->repst, c->rep_upd, c->racc, c->x, c->v,
+                  (const double *)c->mass, (const double *)c->kick, c->pos4, (const long long *)c->f,
+                  (const float *)c->epot, (const float *)c->vir);
 }
 
 void launch_vv_second_b(md_ctx *c, const md_kparams &kp, int energy, int kick)

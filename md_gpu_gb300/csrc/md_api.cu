@@ -381,6 +381,9 @@ md_status capture_graph(md_ctx *c, int nsteps, int energy_first)
     const float4 *start_pos4 = c->pos4;
     if (c->integrator == MD_LEAPFROG && !inl) launch_set_condition(c, (unsigned long long)h[0]);
     int fused = 0;
+    /* a second half and the next first half in one kernel, where nothing
+     * comes between them (no thermostat, no condition to set) */
+    const bool mid = inl && c->integrator == MD_VV;
     for (int k = 0; k < nsteps && s == MD_OK; k++) {
         int energy = (energy_first && k == 0) ? 1 : 0;
         if (c->integrator == MD_LEAPFROG) {
@@ -402,12 +405,13 @@ md_status capture_graph(md_ctx *c, int nsteps, int energy_first)
                 launch_leapfrog(c, kp, energy, hn, has);
             }
         } else {
-            launch_vv_first(c, kp, inl ? 0ull : (unsigned long long)h[k], inl ? 0 : 1);
+            if (k == 0 || !mid) launch_vv_first(c, kp, inl ? 0ull : (unsigned long long)h[k], inl ? 0 : 1);
             if (inl) launch_rebuild(c, kp, false, false, true);
             else s = capture_rebuild_node(c, kp, h[k]);
             if (s != MD_OK) break;
             launch_forces(c, kp, energy != 0, MD_TERM_ALL);
-            launch_vv_second(c, kp, energy);
+            if (mid && k + 1 < nsteps) launch_vv_mid(c, kp, energy);
+            else launch_vv_second(c, kp, energy);
         }
     }
     cudaGraph_t out = nullptr;

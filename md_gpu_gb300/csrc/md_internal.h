@@ -387,6 +387,7 @@ void launch_leapfrog(md_ctx *c, const md_kparams &kp, int energy, unsigned long 
                      int has_cond);
 void launch_vv_first(md_ctx *c, const md_kparams &kp, unsigned long long cond, int has_cond);
 void launch_vv_second(md_ctx *c, const md_kparams &kp, int energy);
+void launch_vv_mid(md_ctx *c, const md_kparams &kp, int energy);
 void launch_thermo_from_state(md_ctx *c, const md_kparams &kp, int energy);
 void launch_gather_out(md_ctx *c, const md_kparams &kp, int what, void *dst);
 void launch_scatter_in(md_ctx *c, const md_kparams &kp, int what, const void *src);
@@ -407,6 +408,7 @@ void launch_leapfrog_b(md_ctx *c, const md_kparams &kp, int energy, unsigned lon
                        int has_cond);
 void launch_vv_first_b(md_ctx *c, const md_kparams &kp, unsigned long long cond, int has_cond);
 void launch_vv_second_b(md_ctx *c, const md_kparams &kp, int energy, int kick);
+void launch_vv_mid_b(md_ctx *c, const md_kparams &kp, int energy);
 
 /* List entries each pair-kernel lane loads per batch for the context's
  * lanes per atom: the autotuner's choice, else the default (TPA * depth
