@@ -190,7 +190,9 @@ md_status md_compute_forces(md_ctx *ctx, int terms, int energy);
 /* nsteps iterations of the reference's loop body (runGPU.cu:69-104):
  * list check and rebuild, forces, integrate.  energy_every > 0 computes
  * energies on steps that are multiples of it (the reference's timprn).
- * Steps run as a captured CUDA graph; no host synchronisation inside.  A
+ * Steps run as captured CUDA graphs, or all in one cooperative launch (steps
+ * without energies of a single system of a few thousand atoms; the same bits);
+ * no host synchronisation inside.  A
  * list rebuild inside the run that finds a row longer than the list holds
  * (the reference writes past its list then, neighborlist.cu:284) truncates
  * rows, so the call saves the state on the device when it starts; after an
@@ -257,7 +259,8 @@ typedef struct {
     int kernels_per_step;   /* kernel launches of one step of a step graph without a rebuild
                                (inline rebuild passes included: they run every step) */
     int kernels_per_rebuild; /* kernels a list rebuild adds to a step (0 with inline passes) */
-    int kernels_per_graph;  /* kernels a step graph runs besides its steps (condition set-up) */
+    int kernels_per_graph;  /* kernels a step graph runs besides its steps (condition set-up;
+                               the first half of a velocity-Verlet graph's first step) */
     int pair_entries_per_lane; /* list entries each pair-kernel lane loads per batch */
     int positions_centered; /* 1: every position uploaded last lay in [-L/2, L/2] per axis,
                                so the fast paths that rely on it are on (the integrators

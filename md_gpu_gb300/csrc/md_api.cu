@@ -2188,10 +2188,11 @@ md_status md_get_info(md_ctx *c, md_info *out)
     out->builds = h.builds;
     out->max_neighbors = *std::max_element(cnt.begin(), cnt.begin() + c->n);
     /* in a step graph without a rebuild: pair, bonded (if any), integrator
-     * (leapfrog: one kernel; VV: two); a rebuild adds 9 kernels */
+     * (leapfrog: one kernel; VV: two, or one where its halves are fused) */
+    const bool mid = md_inline_rebuild(c) && c->integrator == MD_VV;
     out->kernels_per_step = md_can_fuse(c) ? 1
                                            : 1 + ((c->has_bonds || c->has_angles) ? 1 : 0) +
-                                                 (c->integrator == MD_LEAPFROG ? 1 : 2);
+                                                 (c->integrator == MD_LEAPFROG || mid ? 1 : 2);
     /* PME: spread, solve, gather and (with exclusions) the correction, plus
      * the kernels of cuFFT's two transforms, which are not counted */
     if (c->pme.on) out->kernels_per_step += 3 + c->pme.excl;
@@ -2204,7 +2205,7 @@ md_status md_get_info(md_ctx *c, md_info *out)
     if (md_inline_rebuild(c)) {   /* the passes run (and return) in every step */
         out->kernels_per_step += out->kernels_per_rebuild;
         out->kernels_per_rebuild = 0;
-        out->kernels_per_graph = 0;
+        out->kernels_per_graph = mid ? 1 : 0;
     }
     return MD_OK;
 }
