@@ -51,25 +51,33 @@ __global__ void __launch_bounds__(128) k_pair(md_kparams kp, pair_consts pc,
 }
 
 /* Bonds and angles (bonded_atom), one thread per sorted atom, added into the
- * fixed-point forces.
+ * fixed-point forces.  Latency bound (one chain of gathers and an arc cosine
+ * per atom), so it is launched as a programmatic dependent of the pair kernel:
+ * its blocks compute from the positions while that one drains, and wait for it
+ * before they add (every block waits, so that what follows this kernel also
+ * follows the pair kernel).  98304 water atoms: 164.7 -> 161.2 us per step.
  * In a batch (reps non-null) the minimum image uses the atom's replica box. */
 template <bool ENERGY>
-__global__ void k_bonded(md_kparams kp, const float4 *__restrict__ pos4,
+__global__ void __launch_bounds__(256) k_bonded(md_kparams kp, const float4 *pos4,
                          const int2 *__restrict__ bl_s, const int *__restrict__ bl_sn,
                          const int4 *__restrict__ al_s, const int *__restrict__ al_sn,
                          const float *__restrict__ par, int has_bonds, int has_angles,
                          const md_rep *__restrict__ reps, const int *__restrict__ arep,
                          long long *f, float *vir, float *epot)
 {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= kp.n) return;
+    pdl_trigger();   /* the integrator may be scheduled; it waits for this grid */
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const int P = kp.pitch;
-    int nb = has_bonds ? bl_sn[s] : 0;
-    int na = has_angles ? al_sn[s] : 0;
-    if (nb == 0 && na == 0) return;
-    const float *box = reps ? reps[arep[s]].box : kp.box, *boxi = reps ? reps[arep[s]].boxi : kp.boxi;
-    float fx, fy, fz, fw, fe;
-    bonded_atom<ENERGY>(s, P, nb, na, box, boxi, pos4, bl_s, al_s, par, fx, fy, fz, fw, fe);
+    const int nb = s < kp.n && has_bonds ? bl_sn[s] : 0;
+    const int na = s < kp.n && has_angles ? al_sn[s] : 0;
+    const bool any = nb > 0 || na > 0;
+    float fx = 0.0f, fy = 0.0f, fz = 0.0f, fw = 0.0f, fe = 0.0f;
+    if (any) {
+        const float *box = reps ? reps[arep[s]].box : kp.box, *boxi = reps ? reps[arep[s]].boxi : kp.boxi;
+        bonded_atom<ENERGY>(s, P, nb, na, box, boxi, pos4, bl_s, al_s, par, fx, fy, fz, fw, fe);
+    }
+    pdl_wait();   /* the pair forces */
+    if (!any) return;
     f[s] += __float2ll_rn(fx * 4294967296.0f);
     f[P + s] += __float2ll_rn(fy * 4294967296.0f);
     f[2 * P + s] += __float2ll_rn(fz * 4294967296.0f);
@@ -145,13 +153,8 @@ void launch_bonded(md_ctx *c, const md_kparams &kp, bool energy, int terms)
         int nb = (kp.n + 255) / 256;
         const md_rep *reps = c->batch ? c->reps_dev : nullptr;
         const int *arep = c->batch ? c->arep : nullptr;
-        if (energy)
-            k_bonded<true><<<nb, 256, 0, c->stream>>>(kp, c->pos4, c->bl_s, c->bl_sn, c->al_s,
-                                                       c->al_sn, c->bonded_par, hb, ha, reps, arep,
-                                                       c->f, c->vir, c->epot);
-        else
-            k_bonded<false><<<nb, 256, 0, c->stream>>>(kp, c->pos4, c->bl_s, c->bl_sn, c->al_s,
-                                                        c->al_sn, c->bonded_par, hb, ha, reps, arep,
-                                                        c->f, c->vir, c->epot);
+        md_launch_pdl(energy ? k_bonded<true> : k_bonded<false>, dim3(nb), dim3(256), c->stream, kp,
+                      (const float4 *)c->pos4, (const int2 *)c->bl_s, (const int *)c->bl_sn, (const int4 *)c->al_s,
+                      (const int *)c->al_sn, (const float *)c->bonded_par, hb, ha, reps, arep, c->f, c->vir, c->epot);
     }
 }
