@@ -292,27 +292,27 @@ md_status alloc_list(md_ctx *c, int cap)
     return MD_OK;
 }
 
-/* Launch the kernels of `nsteps` steps eagerly (outside a graph): the list
- * kernels return at once unless the previous step's check asked for a build. */
-void enqueue_steps(md_ctx *c, int nsteps, int energy_first)
+/* Launch the kernels of one step eagerly (outside a graph): the list kernels
+ * return at once unless the previous step's check asked for a build.  Velocity
+ * Verlet: first = 0 leaves out the first half (the step before did it), mid = 1
+ * does the next step's with the second half. */
+void enqueue_step(md_ctx *c, int energy, bool first, bool mid)
 {
     md_kparams kp = md_make_kparams(c);
-    for (int k = 0; k < nsteps; k++) {
-        int energy = (energy_first && k == 0) ? 1 : 0;
-        if (c->integrator == MD_LEAPFROG) {
-            launch_rebuild(c, kp, false, false);
-            if (!energy && md_can_fuse(c)) {
-                launch_pair_leapfrog(c, kp, 0, 0);
-            } else {
-                launch_forces(c, kp, energy != 0, MD_TERM_ALL);
-                launch_leapfrog(c, kp, energy, 0, 0);
-            }
+    if (c->integrator == MD_LEAPFROG) {
+        launch_rebuild(c, kp, false, false);
+        if (!energy && md_can_fuse(c)) {
+            launch_pair_leapfrog(c, kp, 0, 0);
         } else {
-            launch_vv_first(c, kp, 0, 0);
-            launch_rebuild(c, kp, false, false);
             launch_forces(c, kp, energy != 0, MD_TERM_ALL);
-            launch_vv_second(c, kp, energy);
+            launch_leapfrog(c, kp, energy, 0, 0);
         }
+    } else {
+        if (first) launch_vv_first(c, kp, 0, 0);
+        launch_rebuild(c, kp, false, false);
+        launch_forces(c, kp, energy != 0, MD_TERM_ALL);
+        if (mid) launch_vv_mid(c, kp, energy);
+        else launch_vv_second(c, kp, energy);
     }
 }
 
@@ -1603,7 +1603,7 @@ static md_status step_body(md_ctx *c, int nsteps, int energy_every, bool mark_st
             continue;
         }
         if (energy_every > 4 && c->host_step % energy_every == 0 && md_can_run_small(c)) {
-            enqueue_steps(c, 1, 1);   /* the energy step between two runs of small steps */
+            enqueue_step(c, 1, true, false);   /* the energy step between two runs of small steps */
             c->host_step++;
             left--;
             continue;
@@ -1617,9 +1617,10 @@ static md_status step_body(md_ctx *c, int nsteps, int energy_every, bool mark_st
                 long long next = (c->host_step / energy_every + 1) * energy_every;
                 k = (int)std::min<long long>(left, next - c->host_step);
             }
+            const bool fuse = c->use_graphs && c->integrator == MD_VV;   /* as in the graphs */
             for (int t = 0; t < k; t++) {
                 int en = energy_every > 0 && (c->host_step % energy_every == 0);
-                enqueue_steps(c, 1, en);
+                enqueue_step(c, en, t == 0 || !fuse, fuse && t + 1 < k);
                 c->host_step++;
             }
             left -= k;

@@ -13,9 +13,10 @@ def _nacl(natom, seed=4, **kw):
     return synth.to_arrays(synth.nacl_replica(natom=natom, seed=seed, **kw))
 
 
-# one step (no middle), an even and an odd run, energies between; the batch
+# one step (no middle), an even and an odd run, one with steps after its last
+# graph, energies between (runs that start between two of them too); the batch
 # has replicas of one block, of a last block of one atom pair and of several
-@pytest.mark.parametrize("steps,every", [(1, 0), (2, 0), (19, 0), (24, 5), (9, 1)])
+@pytest.mark.parametrize("steps,every", [(1, 0), (2, 0), (19, 0), (45, 0), (24, 5), (9, 1)])
 @pytest.mark.parametrize("kind", ["single", "fp64", "batch"])
 def test_fused_halves_match_separate_kernels(kind, steps, every):
     out = []
