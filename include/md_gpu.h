@@ -286,7 +286,8 @@ md_status md_set_tuning(md_ctx *ctx, int pair_tpa, int list_tpa);
  * parallelism against registers): 0 = the default for the lane count (8 for
  * 1-4 lanes, 4 for 8, 2 for 16, 1 for 32); also half the default at 4, 8
  * and 16 lanes.  A new context has 8 lanes and 2 entries, or by its size, a
- * single system of few atoms, 32 or 16 lanes and their default (up to one
+ * single system of few atoms and long rows (128 entries and more expected), 32
+ * or 16 lanes and their default (up to one
  * block of 8 atoms, two of 16 per SM: 1208 and 4848 atoms on 152 SMs; 16 at
  * most with the reciprocal sum);
  * a depth set before any other tuning brings such a context to 8 lanes.

@@ -26,8 +26,8 @@
  *
  * What bounds it is latency: the chain list entry -> position -> force ->
  * update -> barrier of one step, and the rebuilds.  Whole md_step calls of
- * 100 steps against the step graphs: 500 LJ atoms 2.48 -> 0.74 ms, 4000 LJ
- * atoms 2.71 -> 0.96 ms, 982 ions 3.30 -> 1.01 ms; 20 steps of 5184 water
+ * 100 steps against the step graphs: 500 LJ atoms 2.48 -> 0.83 ms, 4000 LJ
+ * atoms 2.71 -> 1.01 ms, 982 ions 3.30 -> 1.01 ms; 20 steps of 5184 water
  * atoms 1.58 -> 0.74 ms.  Above the resident
  * blocks the step graphs are the only form (8000 ions: 16.2 us per step here,
  * 28.4 with 16 lanes per atom, where they do not fit).  Copying the block's
@@ -56,8 +56,8 @@ struct run_thermo {
 
 /* f / 2, exactly (f in 2^-32 kJ/mol/A: a half kick's force).  The step is a
  * chain of FP64 latencies: adding a number whose last place is 1/2 converts
- * and halves in one addition (500 LJ atoms 6.31 -> 6.10 us per step, 4000
- * 7.73 -> 7.28).  Where the FP64 pipe's rate binds instead (the integrator
+ * and halves in one addition (500 LJ atoms at 32 lanes 6.31 -> 6.10 us per
+ * step, 4000 at 16 lanes 7.73 -> 7.28).  Where the FP64 pipe's rate binds instead (the integrator
  * kernels of large systems) the addition costs more than the conversion. */
 __device__ __forceinline__ double half_of(long long f)
 {

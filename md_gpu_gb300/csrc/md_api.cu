@@ -557,16 +557,22 @@ struct host_stage {
  * run of steps in one launch (k_run.cu: blocks of 256 / lanes atoms and one
  * more) has one block per SM at 32 lanes or two at 16, else 8.  A small
  * system's step is a chain of latencies, and more lanes shorten the part of
- * it that walks a row.  us per step at 8 / 16 / 32 lanes: 500 LJ atoms 7.1 /
- * 6.4 / 6.3, 982 ions 12.0 / 9.5 / 9.0, 1536 water atoms 18.5 / 14.4 / 15.4,
- * 2048 LJ atoms 7.6 / 6.5 / 7.5, 4080 ions 12.9 / 11.6 / 26 (too many
- * blocks), 8000 ions 16.2 / 28.4 / - .  With the reciprocal sum, whose kernels
+ * it that walks a row.  us per step at 8 / 16 / 32 lanes: 982 ions 12.0 / 9.5
+ * / 9.0, 1536 water atoms 18.5 / 14.4 / 15.4, 4080 ions 12.9 / 11.6 / 26 (too
+ * many blocks), 8000 ions 16.2 / 28.4 / - .  Rows expected to hold fewer than
+ * 128 entries keep 8 lanes: an LJ liquid's (80 entries at rc 2.5 sigma) gain
+ * less (500 atoms 7.1 / 6.4 / 6.3, 4000 atoms 7.9 / 7.8 / -), and its
+ * trajectories amplify a change in the order of the FP32 sums the most (to
+ * 1e-5 of the velocities in 100 steps).  With the reciprocal sum, whose kernels
  * run beside the pair kernel, 16 at most: 1000 ions 45.5 / 45.0 / 49.0, 2744
  * ions 51.6 / 48.2 / 50.6.  Picked after the first forces, which 8 lanes
  * computed: a context then brought to 8 lanes runs as if it had had them all
  * along. */
 static void pick_lanes(md_ctx *c)
 {
+    const double rl = sqrt((double)c->rskinsq);
+    const double row = c->n * (4.0 / 3.0 * M_PI * rl * rl * rl) / ((double)c->box[0] * c->box[1] * c->box[2]);
+    if (row < 128.0) return;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {

@@ -128,3 +128,8 @@ def test_large_forces_match_separate_kernels():
             out.append((sim.positions(), sim.velocities(), sim.forces()))
     for p, q in zip(*out):
         assert np.array_equal(p, q)
+
+
+def test_short_rows_keep_eight_lanes():
+    with MDSystem.from_arrays(**synth.to_arrays(synth.argon_fcc(ncell=5, seed=3, integrator="vv"))) as sim:
+        assert sim.info()["pair_tpa"] == 8 and sim.info()["pair_depth"] == 2
