@@ -711,7 +711,7 @@ extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const 
         if (v) launch_gather_out(c, kp, 1, v);
     };
     /* one VV step, the list forced at checkpoint frames */
-    auto step = [&](int s_idx, bool energy) {   /* the same forces with and without energies */
+    auto step = [&](int s_idx, bool energy) {
         launch_vv_first(c, kp, 0, 0);
         launch_rebuild(c, kp, (s_idx + 1) % C == 0, (s_idx + 1) % C == 0);
         launch_forces(c, kp, energy, MD_TERM_ALL);
@@ -789,8 +789,9 @@ extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const 
     if (keep)
         for (int m = K; m >= 0; m--) back(m, B.seg + n3 * m);
     /* forces without energies have the same bits where entries are evaluated
-     * two at a time and there are no bonded terms */
-    const bool energy2 = md_pair_depth(c) % 2 != 0 || c->has_bonds || c->has_angles;
+     * two at a time with energies too (the Wolf form) and there are no bonded
+     * terms */
+    const bool energy2 = c->lkspace == 0 || md_pair_depth(c) % 2 != 0 || c->has_bonds || c->has_angles;
     for (int sg = nseg - 1; sg >= 0 && !keep; sg--) {
         const int m0 = sg * C, m1 = std::min(K, m0 + C);
         /* recompute the segment from its checkpoint, as the forward run did */

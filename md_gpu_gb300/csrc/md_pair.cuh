@@ -228,7 +228,8 @@ struct wrap2 {
  * vary per entry run on v2; those with a per-atom or per-system constant run
  * as scalar IEEE operations with the constant (no register pair to hold it).
  * The same formulas as pair_term, with every rounding step fixed, and the
- * same forces with and without ENERGY. */
+ * same forces with and without ENERGY (pair_sum takes it for the Wolf form
+ * then). */
 template <int KIND, bool ENERGY, bool WRAP, bool PACKED, class G>
 __device__ __forceinline__ void pair_term2(const G &g, const wrap2<PACKED> &W, v2<PACKED> PX, v2<PACKED> PY,
                                            v2<PACKED> PZ, float qi, float4 p0, float4 p1, float2 l0,
@@ -447,6 +448,10 @@ __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool
                                                const int *nl_n, const float2 *lj)
 {
     static_assert(MD_LIST_QUANTUM % (TPA * B) == 0, "batch must divide the list padding");
+    /* LJ and reaction field sum one entry at a time where energies are asked
+     * for: an LJ liquid amplifies a change in the order of the sums the most,
+     * and its energy steps are short (500 to 4000 atoms: 6 us) */
+    constexpr bool PK = PACK && (KIND == 1 || !ENERGY);
     const float4 pi = pos4[ii];
     const int cnt = active ? nl_n[ii] : 0;
     /* batches of TPA * B entries up to the first that holds the row's last
@@ -464,9 +469,9 @@ __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool
     const bool inner = g.centered() && __all_sync(0xffffffffu, !active || interior(g, pi));
     if (nb > 0) {
         if (inner)
-            pair_loop<KIND, TPA, B, ENERGY, false, PACK, SETS, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
+            pair_loop<KIND, TPA, B, ENERGY, false, PK, SETS, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
         else
-            pair_loop<KIND, TPA, B, ENERGY, true, PACK, SETS, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
+            pair_loop<KIND, TPA, B, ENERGY, true, PK, SETS, NC>(g, pi, qi, nb, lp, pos4, ljrow, acc);
     }
     pair_total r;
     r.fx = __float2ll_rn(acc.fx * 4294967296.0f);

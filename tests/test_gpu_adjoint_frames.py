@@ -1,6 +1,6 @@
 """The adjoint over kept frames against the one that runs the trajectory again
-from checkpoints, and the property the latter rests on: pair forces have the
-same bits with and without energies."""
+from checkpoints, and the property the latter rests on: pair forces of the Wolf
+form have the same bits with and without energies."""
 import numpy as np
 import pytest
 
@@ -15,11 +15,15 @@ def _reps(sizes):
 
 
 # one atom past a 16-atom block; segments that do and do not divide the run
-@pytest.mark.parametrize("sizes,steps,checkpoint", [((514,), 12, 4), ((512, 978), 11, 5), ((998, 510, 512), 7, 7)])
-def test_kept_frames_match_recompute(sizes, steps, checkpoint):
+@pytest.mark.parametrize("lkspace,sizes,steps,checkpoint", [
+    (1, (514,), 12, 4), (1, (512, 978), 11, 5), (1, (998, 510, 512), 7, 7), (0, (512, 514), 11, 5)])
+def test_kept_frames_match_recompute(lkspace, sizes, steps, checkpoint):
     out = []
+    reps = _reps(sizes)
+    for a in reps:
+        a.update(lkspace=lkspace, reacf=1e-3 if lkspace == 0 else 0.0)
     for keep in (1, 0):
-        with MDSystem.from_batch(_reps(sizes)) as sim:
+        with MDSystem.from_batch(reps) as sim:
             assert library().md_debug_adjoint_frames(sim._ctx, keep) == 0
             o = sim.adjoint(steps, checkpoint=checkpoint, nbins=100)
             out.append((o, sim.positions(), sim.velocities()))
@@ -32,13 +36,10 @@ def test_kept_frames_match_recompute(sizes, steps, checkpoint):
         assert np.abs(a[k] - b[k]).max() <= 2e-5 * np.abs(a[k]).max()
 
 
-@pytest.mark.parametrize("lkspace", [0, 1])
 @pytest.mark.parametrize("batch", [False, True])
 @pytest.mark.parametrize("tpa,depth", [(8, 2), (8, 4), (4, 4), (16, 2)])
-def test_forces_same_with_energies(lkspace, batch, tpa, depth):
+def test_forces_same_with_energies(batch, tpa, depth):
     reps = _reps((998, 1728))
-    for a in reps:
-        a.update(lkspace=lkspace, reacf=1e-3 if lkspace == 0 else 0.0)
     sim = MDSystem.from_batch(reps) if batch else MDSystem.from_arrays(**reps[1])
     with sim:
         sim.set_tuning(tpa, 0, depth)
