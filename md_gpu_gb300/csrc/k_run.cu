@@ -217,7 +217,10 @@ __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pai
         return moved;
     };
     __syncthreads();   /* lj and s_ts are set */
-    int flag = a.vv ? 0 : *(volatile int *)&st->update;
+    /* a request left by the step before, or by whoever changed the list
+     * since (the same in every block: cleared by a rebuild only, after the
+     * first barrier) */
+    int flag = *(volatile int *)&st->update;
     if (a.vv) {
         /* first half of the first step, from the forces in memory */
         if (upd) {
@@ -226,7 +229,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pai
         }
         const bool moved = drift();
         if (!barrier(0, -1, true, moved)) return;
-        flag = s_flag;
+        flag |= s_flag;
     }
     for (int k = 0; k < a.nsteps; k++) {
         if (flag) {
