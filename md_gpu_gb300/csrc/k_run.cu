@@ -325,15 +325,26 @@ __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pai
     }
 }
 
+/* The kernel for the context's lanes and entries per lane, null where there
+ * is none.  Four entries per lane go two at a time like two, with the same
+ * sums; one (16 lanes) goes one at a time, rounded otherwise. */
 template <int KIND>
-const void *run_kernel(int tpa)
+const void *run_kernel(int tpa, int depth)
 {
-    switch (tpa) {
-    case 8: return (const void *)k_run_steps<KIND, 8, 2>;
-    case 16: return (const void *)k_run_steps<KIND, 16, 2>;
-    case 32: return (const void *)k_run_steps<KIND, 32, 1>;
+    switch (tpa * 100 + depth) {
+    case 802:
+    case 804: return (const void *)k_run_steps<KIND, 8, 2>;
+    case 1601: return (const void *)k_run_steps<KIND, 16, 1>;
+    case 1602: return (const void *)k_run_steps<KIND, 16, 2>;
+    case 3201: return (const void *)k_run_steps<KIND, 32, 1>;
     default: return nullptr;
     }
+}
+
+const void *run_kernel(const md_ctx *c)
+{
+    const int depth = md_pair_depth(c);
+    return c->lkspace == 0 ? run_kernel<0>(c->pair_tpa, depth) : run_kernel<1>(c->pair_tpa, depth);
 }
 
 }  // namespace
@@ -346,15 +357,16 @@ const void *run_kernel(int tpa)
 bool md_can_run_small(md_ctx *c)
 {
     if (c->batch || c->fp64 || c->pme.on || !c->use_graphs || c->dbg_bar_ns || c->dbg_bar_drop >= 0) return false;
-    const void *k = c->lkspace == 0 ? run_kernel<0>(c->pair_tpa) : run_kernel<1>(c->pair_tpa);
+    const void *k = run_kernel(c);
     if (!k || !md_rebuild_coop(c)) return false;
-    if (c->run_key != c->pair_tpa) {   /* resident blocks, found once per lane count */
+    const int key = c->pair_tpa * 100 + md_pair_depth(c);
+    if (c->run_key != key) {   /* resident blocks, found once per kernel */
         int dev = 0, nsm = 0, occ = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, RUN_THREADS, 0);
         c->run_blocks = nsm * occ;
-        c->run_key = c->pair_tpa;
+        c->run_key = key;
     }
     const int na = RUN_THREADS / c->pair_tpa;
     return (c->n + na - 1) / na + 1 <= c->run_blocks;
@@ -385,8 +397,7 @@ bool launch_run_steps(md_ctx *c, const md_kparams &kp0, int nsteps)
     const int na = RUN_THREADS / c->pair_tpa, blocks = (c->n + na - 1) / na + 1;
     rb_ptrs p = make_rb_ptrs(c, blocks);
     void *args[] = {&kp, &pc, &tp, &a, &p};
-    const void *k = c->lkspace == 0 ? run_kernel<0>(c->pair_tpa) : run_kernel<1>(c->pair_tpa);
-    if (cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(RUN_THREADS), args, 0, c->stream) !=
+    if (cudaLaunchCooperativeKernel(run_kernel(c), dim3(blocks), dim3(RUN_THREADS), args, 0, c->stream) !=
         cudaSuccess) {
         (void)cudaGetLastError();
         return false;

@@ -262,7 +262,7 @@ struct md_ctx {
     int nsm = 1;                   /* SMs of the device (found with cw_grid) */
     unsigned long long *run_ctl = nullptr; /* barrier and sums of k_run_steps: two sets of 64 words */
     int run_parity = 0;            /* the set its next launch uses */
-    int run_key = 0, run_blocks = 0; /* resident blocks of k_run_steps and the lane count they are for */
+    int run_key = 0, run_blocks = 0; /* resident blocks of k_run_steps and the kernel (100 lanes + depth) they are for */
     int rebuild_inline = 0;        /* step graphs: 1 = list passes inline (programmatic launches
                                       that return at once without a request), 0 = a conditional node */
     long long host_step = 0;       /* steps run so far (mirrors st->step) */

@@ -440,8 +440,9 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
  * pair_term2 as packed f32x2 instructions (each lane keeping even- and
  * odd-entry sums); otherwise one at a time through pair_term.  Each lane sums in
  * FP32 and converts its sum to int64 once; lane sums are combined with
- * integer shuffles (exact), so the result depends only on TPA.  Every lane of
- * the warp must call this (the shuffles use the full mask). */
+ * integer shuffles (exact), so the result depends on TPA and on whether B is
+ * even only.  Every lane of the warp must call this (the shuffles use the full
+ * mask). */
 template <int KIND, int TPA, int B, bool ENERGY, bool PACK = true, int SETS = 1, bool NC = true, class G>
 __device__ __forceinline__ pair_total pair_sum(const G &g, int cap, int ii, bool active, int lane,
                                                const float4 *pos4, const int *type, const unsigned *nl,
