@@ -2,9 +2,10 @@
  * k_pair64.cu -- the FP64 mode of the force kernels (md_set_precision(ctx,
  * 64)): the same pair and bonded force laws as the FP32 kernels, evaluated
  * in FP64 on the FP64 positions.  Pair forces without energies take the
- * Coulomb term from a piecewise polynomial within 4e-15 of it and 1/r from
- * an iteration (rsqrt64); energies and bonded terms use exp, log and IEEE
- * divide and square root.
+ * Coulomb term from a piecewise polynomial within 1e-16 of it and 1/r from
+ * an iteration (rsqrt64), which together come closer to the force law than
+ * FP64 arithmetic on the form as written; energies and bonded terms use exp,
+ * log and IEEE divide and square root.
  *
  * This is the "plain FP64" form of the path run on the GPU: the reference
  * point of the precision gates (RMS force error, NVE drift) and the per-system
@@ -44,7 +45,9 @@ struct md_p64_model {
 
 /* 1 / sqrt(s) for s in FP32's normal range: the FP32 approximation and one
  * step of Halley's iteration, whose error is about e^3 / 3 for a seed of
- * relative error e / 2 ~ 2^-23; two roundings of the FP64 result remain. */
+ * relative error e / 2 ~ 2^-23.  y y is exact (48 bits) and e rounded once,
+ * so what remains is the rounding of the result: half an ulp and 2^-22 of
+ * one, against one ulp for a square root and a divide. */
 __device__ __forceinline__ double rsqrt64(double s, float &seed)
 {
     seed = rsqrt_approx((float)s);
@@ -58,25 +61,28 @@ __device__ __forceinline__ double rsqrt64(double s, float &seed)
  * instruction in 20 cycles, so its operations are what counts: without
  * energies the Coulomb term comes from a piecewise polynomial (tab, 8 FP64
  * operations; exp and the divide of the A&S form take over 40).  4082 ions,
- * per launch: 230 us before, 102 us now (80% of the FP64 pipe), the error of
- * eight velocity-Verlet steps against 64 bits unchanged (6.4e-13). */
+ * per launch: 230 us as written, 102 us so.  Its argument r - centre is one
+ * fma of r^2 and 1/r: r itself is never rounded.  Against quad precision, at
+ * distances from 1.5 A to rc (a rc 0.5 to 3.2): the largest error of G 1.2e-16
+ * to 2.3e-16 (rms 4e-17), the form as written in FP64 4.1e-16 to 7.7e-16 (rms
+ * 6e-17 to 1.8e-16). */
 template <int KIND, bool ENERGY>
-__device__ __forceinline__ void pair64_eval(const md_p64_model &m, const double (*tab)[MD_P64_DEG + 2], double rsq,
+__device__ __forceinline__ void pair64_eval(const md_p64_model &m, const double *tab, double rsq,
                                             double qq, double lja, double ljc, double &ff, double &u)
 {
     float seed;
-    const double ri = rsqrt64(rsq, seed), r = rsq * ri, ri2 = ri * ri;
+    const double ri = rsqrt64(rsq, seed), ri2 = ri * ri;
     double fc, uc = 0.0;
     if (KIND == 1) {
         if (!ENERGY && m.ni > 0) {
-            const double *c = tab[min((int)((float)rsq * seed * m.nih), m.ni - 1)];
-            const double y = r - c[0];
+            const double *c = tab + (MD_P64_DEG + 2) * min((int)((float)rsq * seed * m.nih), m.ni - 1);
+            const double y = fma(rsq, ri, -c[0]);
             double g = c[MD_P64_DEG + 1];
 #pragma unroll
             for (int k = MD_P64_DEG; k > 0; k--) g = fma(g, y, c[k]);
             fc = qq * fma(g, ri, -m.wolfw);
         } else {
-            const double xa = m.alpha * r;
+            const double r = sqrt(rsq), xa = m.alpha * r;
             const double t = 1.0 / (1.0 + m.pex * xa);
             const double p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
             const double ex = exp(-xa * xa);
@@ -112,7 +118,7 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
                                                        float *vir, float *epot)
 {
     __shared__ double2 lj[MD_MAXTYPE * MD_MAXTYPE];
-    __shared__ double s_g[MD_P64_MAXI][MD_P64_DEG + 2];
+    extern __shared__ double s_g[];   /* the replica's table */
     pdl_trigger();   /* the integrator may be scheduled; it waits for this grid */
     int rep = 0, i0, end;
     if (tab) {
@@ -147,7 +153,7 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
         }
         if (KIND == 1 && !ENERGY) {
             const double *g = &M.g[0][0];
-            for (int k = threadIdx.x; k < m.ni * (MD_P64_DEG + 2); k += blockDim.x) (&s_g[0][0])[k] = g[k];
+            for (int k = threadIdx.x; k < m.ni * (MD_P64_DEG + 2); k += blockDim.x) s_g[k] = g[k];
         }
     }
     for (int k = threadIdx.x; k < MD_MAXTYPE * MD_MAXTYPE; k += blockDim.x) {
@@ -323,54 +329,55 @@ __global__ void k_bonded64(int n, int pitch, const double *__restrict__ boxd,
 
 /* The pieces of G(r) = E(r) + spi r e^{-a^2 r^2} on [0, rc], E(r) = P5(t) t
  * e^{-a^2 r^2}, t = 1 / (1 + p a r): on each the Chebyshev interpolant of
- * degree MD_P64_DEG, written in powers of r - centre.  Takes the fewest
- * pieces whose largest deviation at 16 points a piece is at most 4e-15 (G is
- * about 1 or less; FP64 evaluation of the form as written is no closer);
- * none: m.ni = 0. */
+ * degree MD_P64_DEG, written in powers of r - centre and computed in long
+ * double, so that its coefficients are as good as FP64 holds them.  Takes the
+ * fewest pieces whose largest deviation at 16 points a piece is at most 1e-16,
+ * an ulp of G just below 1 (G as written, evaluated in FP64, is off by 4e-16
+ * to 8e-16; at 4e-15, the line before, the pieces were the larger error); none:
+ * m.ni = 0. */
 static void fit_coulomb(md_p64 &m)
 {
-    constexpr int N = MD_P64_DEG + 1;
-    auto G = [&](double r) {
-        const double xa = m.alpha * r, t = 1.0 / (1.0 + m.pex * xa);
-        const double p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
-        const double ex = exp(-xa * xa);
+    typedef long double real;
+    constexpr int N = MD_P64_DEG + 1, CHK = 16;
+    auto G = [&](real r) {
+        const real xa = m.alpha * r, t = 1.0L / (1.0L + m.pex * xa);
+        const real p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
+        const real ex = expl(-xa * xa);
         return p * t * ex + m.spi * r * ex;
     };
-    const double pi = 3.14159265358979323846;
+    const real pi = acosl(-1.0L);
+    /* T_j at the nodes, weighted, and (monomial) T_j's coefficients */
+    real node[N], tj[N][N], mono[N][N] = {};
+    for (int k = 0; k < N; k++) {
+        node[k] = cosl(pi * (k + 0.5L) / N);
+        for (int j = 0; j < N; j++) tj[j][k] = cosl(pi * j * (k + 0.5L) / N) * (j == 0 ? 1.0L : 2.0L) / N;
+    }
+    mono[0][0] = mono[1][1] = 1.0L;
+    for (int j = 2; j < N; j++)
+        for (int k = 0; k < N; k++) mono[j][k] = (k > 0 ? 2.0L * mono[j - 1][k - 1] : 0.0L) - mono[j - 2][k];
     for (int ni = 16; ni <= MD_P64_MAXI; ni *= 2) {
         const double h = 0.5 * m.rc / ni;   /* half a piece */
-        double worst = 0.0;
-        for (int q = 0; q < ni; q++) {
+        bool ok = true;
+        for (int q = 0; q < ni && ok; q++) {
             const double cen = (2 * q + 1) * h;
-            double f[N], mono[N] = {0.0}, tp[N] = {0.0}, tc[N] = {0.0};
-            for (int k = 0; k < N; k++) f[k] = G(cen + h * cos(pi * (k + 0.5) / N));
+            real f[N], c[N] = {};
+            for (int k = 0; k < N; k++) f[k] = G(cen + h * node[k]);
             for (int j = 0; j < N; j++) {
-                double a = 0.0;
-                for (int k = 0; k < N; k++) a += f[k] * cos(pi * j * (k + 0.5) / N);
-                a *= (j == 0 ? 1.0 : 2.0) / N;
-                /* tc = T_j in powers: T_0 = 1, T_1 = y, T_j = 2 y T_{j-1} - T_{j-2} */
-                double tn[N] = {0.0};
-                if (j == 0) tn[0] = 1.0;
-                else if (j == 1) tn[1] = 1.0;
-                else
-                    for (int k = 0; k < N; k++) tn[k] = (k > 0 ? 2.0 * tc[k - 1] : 0.0) - tp[k];
-                for (int k = 0; k < N; k++) {
-                    mono[k] += a * tn[k];
-                    tp[k] = tc[k];
-                    tc[k] = tn[k];
-                }
+                real a = 0.0L;
+                for (int k = 0; k < N; k++) a += f[k] * tj[j][k];
+                for (int k = 0; k <= j; k++) c[k] += a * mono[j][k];
+            }
+            for (int k = 0; k < CHK && ok; k++) {
+                const real y = -1.0L + (2 * k + 1) / (real)CHK;
+                real g = 0.0L;
+                for (int d = N - 1; d >= 0; d--) g = g * y + c[d];
+                ok = fabsl(g - G(cen + h * y)) <= 1e-16L;
             }
             m.g[q][0] = cen;
-            double hk = 1.0;
-            for (int k = 0; k < N; k++, hk *= h) m.g[q][k + 1] = mono[k] / hk;
-            for (int k = 0; k < 16; k++) {
-                const double y = h * (-1.0 + (2 * k + 1) / 16.0);
-                double g = m.g[q][N];
-                for (int d = N - 1; d > 0; d--) g = g * y + m.g[q][d];
-                worst = std::max(worst, fabs(g - G(cen + y)));
-            }
+            real hk = 1.0L;
+            for (int k = 0; k < N; k++, hk *= h) m.g[q][k + 1] = (double)(c[k] / hk);
         }
-        if (worst <= 4e-15) {
+        if (ok) {
             m.ni = ni;
             m.nih = (float)(ni / m.rc);
             return;
@@ -381,8 +388,10 @@ static void fit_coulomb(md_p64 &m)
 
 /* FP64 model constants of one system (pairmodel of the plain form): rc from
  * the FP32 rc^2 as given, the Wolf shift and energy constants with the A&S
- * erfc in FP64. */
-md_p64 md_make_p64(int lkspace, float rcutsq, float reacf, float alfa, const float box[3])
+ * erfc in FP64.  The table is that of one of the nmade models made before it
+ * with the same rc and alpha, if there is one (a fit takes milliseconds). */
+md_p64 md_make_p64(int lkspace, float rcutsq, float reacf, float alfa, const float box[3], const md_p64 *made,
+                   int nmade)
 {
     md_p64 m;
     memset(&m, 0, sizeof(m));
@@ -416,7 +425,15 @@ md_p64 md_make_p64(int lkspace, float rcutsq, float reacf, float alfa, const flo
     } else if (lkspace == 0) {
         m.ucc = 1.0 / m.rc + 0.5 * m.reacf * m.rcsq;
     }
-    if (lkspace != 0) fit_coulomb(m);
+    if (lkspace == 0) return m;
+    for (int k = 0; k < nmade; k++)
+        if (made[k].rcsq == m.rcsq && made[k].alpha == m.alpha) {
+            m.ni = made[k].ni;
+            m.nih = made[k].nih;
+            memcpy(m.g, made[k].g, sizeof(m.g));
+            return m;
+        }
+    fit_coulomb(m);
     return m;
 }
 
@@ -432,6 +449,7 @@ void launch_pair64(md_ctx *c, bool energy)
      * two and some with one, 116 us per launch; 102 us with one warp) */
     const int atoms = c->n / (P64_THREADS / P64_TPA) < 16 * nsm ? 32 / P64_TPA : P64_THREADS / P64_TPA;
     const int threads = atoms * P64_TPA;
+    const size_t table = sizeof(double) * (MD_P64_DEG + 2) * (size_t)c->p64_ni;   /* the largest of the replicas' */
     if (batch) {
         const int k = md_grid_index(atoms);
         tab = c->grid_tab + c->grid_off[k];
@@ -450,7 +468,7 @@ void launch_pair64(md_ctx *c, bool energy)
         else k_pair64<0, false><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
     } else {
         if (energy) k_pair64<1, true><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
-        else k_pair64<1, false><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
+        else k_pair64<1, false><<<nb, threads, table, c->stream>>>(MD_P64_ARGS);
     }
 #undef MD_P64_ARGS
 }

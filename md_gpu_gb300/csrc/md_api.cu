@@ -2461,10 +2461,11 @@ md_status md_set_precision(md_ctx *c, int bits)
         for (int r = 0; r < nm; r++) {
             if (c->batch) {
                 const md_rep &R = c->reps[r];
-                h[r] = md_make_p64(c->lkspace, R.rcutsq, R.reacf, c->rep_alfa[r], R.box);
+                h[r] = md_make_p64(c->lkspace, R.rcutsq, R.reacf, c->rep_alfa[r], R.box, h.data(), r);
             } else {
-                h[r] = md_make_p64(c->lkspace, c->rcutsq, c->reacf, c->alfa, c->box);
+                h[r] = md_make_p64(c->lkspace, c->rcutsq, c->reacf, c->alfa, c->box, nullptr, 0);
             }
+            c->p64_ni = std::max(c->p64_ni, h[r].ni);
         }
         MD_CUDA_TRY(c, dalloc(&c->p64_dev, (size_t)nm));
         MD_CUDA_TRY(c, cudaMemcpy(c->p64_dev, h.data(), sizeof(md_p64) * nm, cudaMemcpyHostToDevice));

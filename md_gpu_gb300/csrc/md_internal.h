@@ -122,7 +122,7 @@ struct md_rep {
  * md_set_precision): cutoff, reaction-field or Wolf constants, the A&S erfc
  * coefficients widened from the reference's floats, box. */
 constexpr int MD_P64_DEG = 7;     /* degree of a piece of the tabulated Coulomb term */
-constexpr int MD_P64_MAXI = 64;   /* pieces, at most */
+constexpr int MD_P64_MAXI = 128;  /* pieces, at most */
 struct md_p64 {
     int kind;   /* lkspace: 0 reaction field, 1 Wolf, 2 LJ + no Coulomb shift */
     int ni;     /* pieces of G(r) = E(r) + 2 a r / sqrt(pi) e^{-a^2 r^2} on [0, rc], E the A&S
@@ -133,7 +133,8 @@ struct md_p64 {
     double rcsq, rc, rcinv, rc6i, reacf, alpha, spi, pex, a[5], qfac, wolfw, ucc;
     double L[3], Li[3];
 };
-md_p64 md_make_p64(int lkspace, float rcutsq, float reacf, float alfa, const float box[3]);
+md_p64 md_make_p64(int lkspace, float rcutsq, float reacf, float alfa, const float box[3], const md_p64 *made,
+                   int nmade);
 
 /* Per-replica thermodynamic state of a batch (the fields md_devstate holds
  * for a single system). */
@@ -280,6 +281,7 @@ struct md_ctx {
     int fp64 = 0;        /* 1: force kernels in FP64 on the FP64 positions (md_set_precision) */
     double baro[3] = {1.0, 1000.0, 4.5e-5};   /* NPT: target bar, tau_p fs, compressibility 1/bar */
     md_p64 *p64_dev = nullptr;        /* FP64 model constants per replica (1 for a single system) */
+    int p64_ni = 0;                   /* pieces of the largest of their tables */
     std::vector<float> rep_alfa;      /* damping alpha per replica of a batch */
 
     /* batches of replicas (md_create_batch; any number, 1 included) */
