@@ -312,8 +312,8 @@ md_status md_set_type_exclusions(md_ctx *ctx, const unsigned *mask);
  * FP32 on the FP32 copy of the positions, as the reference's kernels do
  * (pair_forces.cu:34-205); 64 evaluates pair, bond and angle terms in FP64
  * on the FP64 positions (the plain FP64 form of the same force law, A&S erfc
- * included; the Coulomb term of pair forces without energies from a
- * piecewise polynomial within 1e-16 of it).  Forces, integrators and
+ * included; the Coulomb term of pair forces from a piecewise polynomial within
+ * 1e-16 of it; the same bits with and without energies).  Forces, integrators and
  * reductions are shared (int64 fixed-point forces, FP64 state).  No
  * counterpart in the reference; the FP64 mode is the GPU reference point of
  * the precision checks.  Recomputes the forces of the current state.  FP64

@@ -1,7 +1,7 @@
 /*
  * k_pair64.cu -- the FP64 mode of the force kernels (md_set_precision(ctx,
  * 64)): the same pair and bonded force laws as the FP32 kernels, evaluated
- * in FP64 on the FP64 positions.  Pair forces without energies take the
+ * in FP64 on the FP64 positions.  Pair forces take the
  * Coulomb term from a piecewise polynomial within 1e-16 of it and 1/r from
  * an iteration (rsqrt64), which together come closer to the force law than
  * FP64 arithmetic on the form as written; energies and bonded terms use exp,
@@ -58,44 +58,52 @@ __device__ __forceinline__ double rsqrt64(double s, float &seed)
 
 /* One pair: ff (F_i = ff d) and the pair energy (consistent potential,
  * LJ shifted to zero at rc) for r^2 <= rc^2.  The FP64 pipe issues one warp
- * instruction in 20 cycles, so its operations are what counts: without
- * energies the Coulomb term comes from a piecewise polynomial (tab, 8 FP64
- * operations; exp and the divide of the A&S form take over 40).  4082 ions,
+ * instruction in 20 cycles, so its operations are what counts: the force's
+ * Coulomb term comes from a piecewise polynomial (tab, 8 FP64 operations;
+ * exp and the divide of the A&S form, which the energy takes, over 40).  4082 ions,
  * per launch: 230 us as written, 102 us so.  Its argument r - centre is one
  * fma of r^2 and 1/r: r itself is never rounded.  Against quad precision, at
  * distances from 1.5 A to rc (a rc 0.5 to 3.2): the largest error of G 1.2e-16
  * to 2.3e-16 (rms 4e-17), the form as written in FP64 4.1e-16 to 7.7e-16 (rms
- * 6e-17 to 1.8e-16). */
+ * 6e-17 to 1.8e-16).  Every rounding of the force is written out (no
+ * contraction is left to the compiler), so that it has the same bits with and
+ * without ENERGY and a trajectory does not depend on its energy steps. */
 template <int KIND, bool ENERGY>
 __device__ __forceinline__ void pair64_eval(const md_p64_model &m, const double *tab, double rsq,
                                             double qq, double lja, double ljc, double &ff, double &u)
 {
     float seed;
-    const double ri = rsqrt64(rsq, seed), ri2 = ri * ri;
+    const double ri = rsqrt64(rsq, seed), ri2 = __dmul_rn(ri, ri);
     double fc, uc = 0.0;
     if (KIND == 1) {
-        if (!ENERGY && m.ni > 0) {
+        const bool table = m.ni > 0;
+        double ec = 0.0, ex = 0.0, r = 0.0;
+        if (ENERGY || !table) {   /* the form as written */
+            r = __dmul_rn(rsq, ri);
+            r = fma(fma(-r, r, rsq), __dmul_rn(0.5, ri), r);
+            const double xa = __dmul_rn(m.alpha, r);
+            const double t = __ddiv_rn(1.0, fma(m.pex, xa, 1.0));
+            const double p = fma(fma(fma(fma(m.a[4], t, m.a[3]), t, m.a[2]), t, m.a[1]), t, m.a[0]);
+            ex = exp(-__dmul_rn(xa, xa));
+            ec = __dmul_rn(__dmul_rn(p, t), ex);
+        }
+        if (table) {
             const double *c = tab + (MD_P64_DEG + 2) * min((int)((float)rsq * seed * m.nih), m.ni - 1);
             const double y = fma(rsq, ri, -c[0]);
             double g = c[MD_P64_DEG + 1];
 #pragma unroll
             for (int k = MD_P64_DEG; k > 0; k--) g = fma(g, y, c[k]);
-            fc = qq * fma(g, ri, -m.wolfw);
+            fc = __dmul_rn(qq, fma(g, ri, -m.wolfw));
         } else {
-            const double r = sqrt(rsq), xa = m.alpha * r;
-            const double t = 1.0 / (1.0 + m.pex * xa);
-            const double p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
-            const double ex = exp(-xa * xa);
-            const double ec = p * t * ex;
-            fc = qq * ((ec * ri + m.spi * ex) - m.wolfw);
-            if (ENERGY) uc = qq * (ec * ri - m.ucc + m.wolfw * log(r * m.rcinv));
+            fc = __dmul_rn(qq, __dsub_rn(fma(ec, ri, __dmul_rn(m.spi, ex)), m.wolfw));
         }
+        if (ENERGY) uc = qq * (ec * ri - m.ucc + m.wolfw * log(r * m.rcinv));
     } else {
-        fc = qq * (ri - m.reacf * rsq);
+        fc = __dmul_rn(qq, fma(-m.reacf, rsq, ri));
         if (ENERGY) uc = qq * (ri + 0.5 * m.reacf * rsq - m.ucc);
     }
-    const double ri6 = ri2 * ri2 * ri2;
-    ff = ri2 * (fc + ri6 * (lja * ri6 - ljc));
+    const double ri6 = __dmul_rn(__dmul_rn(ri2, ri2), ri2);
+    ff = __dmul_rn(ri2, fma(ri6, fma(lja, ri6, -ljc), fc));
     if (ENERGY)
         u = uc + (lja * (1.0 / 12.0) * (ri6 * ri6 - m.rc6i * m.rc6i) - ljc * (1.0 / 6.0) * (ri6 - m.rc6i));
 }
@@ -151,7 +159,7 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
             m.L[k] = M.L[k];
             m.Li[k] = M.Li[k];
         }
-        if (KIND == 1 && !ENERGY) {
+        if (KIND == 1) {
             const double *g = &M.g[0][0];
             for (int k = threadIdx.x; k < m.ni * (MD_P64_DEG + 2); k += blockDim.x) s_g[k] = g[k];
         }
@@ -195,19 +203,19 @@ __global__ void __launch_bounds__(P64_THREADS) k_pair64(int n, int pitch, int ca
             if (ny != 0.0f) dy = fma(-m.L[1], (double)ny, dy);
             if (nz != 0.0f) dz = fma(-m.L[2], (double)nz, dz);
         } else if (!inner) {
-            dx -= m.L[0] * rint(dx * m.Li[0]);
-            dy -= m.L[1] * rint(dy * m.Li[1]);
-            dz -= m.L[2] * rint(dz * m.Li[2]);
+            dx = fma(-m.L[0], rint(__dmul_rn(dx, m.Li[0])), dx);
+            dy = fma(-m.L[1], rint(__dmul_rn(dy, m.Li[1])), dy);
+            dz = fma(-m.L[2], rint(__dmul_rn(dz, m.Li[2])), dz);
         }
-        const double rsq = dx * dx + dy * dy + dz * dz;
+        const double rsq = fma(dz, dz, fma(dy, dy, __dmul_rn(dx, dx)));
         if (rsq <= m.rcsq && (float)rsq > 0.0f) {
             const double2 l = ljrow[e >> MD_TYPE_SHIFT];
             double ff, u = 0.0;
-            pair64_eval<KIND, ENERGY>(m, s_g, rsq, qi * (double)pj.w, l.x, l.y, ff, u);
-            fx += ff * dx;
-            fy += ff * dy;
-            fz += ff * dz;
-            fw += ff * rsq;
+            pair64_eval<KIND, ENERGY>(m, s_g, rsq, __dmul_rn(qi, (double)pj.w), l.x, l.y, ff, u);
+            fx = fma(ff, dx, fx);
+            fy = fma(ff, dy, fy);
+            fz = fma(ff, dz, fz);
+            fw = fma(ff, rsq, fw);
             if (ENERGY) fe += 0.5 * u;
         }
     }
@@ -467,7 +475,7 @@ void launch_pair64(md_ctx *c, bool energy)
         if (energy) k_pair64<0, true><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
         else k_pair64<0, false><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
     } else {
-        if (energy) k_pair64<1, true><<<nb, threads, 0, c->stream>>>(MD_P64_ARGS);
+        if (energy) k_pair64<1, true><<<nb, threads, table, c->stream>>>(MD_P64_ARGS);
         else k_pair64<1, false><<<nb, threads, table, c->stream>>>(MD_P64_ARGS);
     }
 #undef MD_P64_ARGS

@@ -72,7 +72,7 @@ def _forces(sim, pos, energy):
 # a rc from 0.5 to 3.5 (16 to 128 pieces), the real-space Ewald form, and one without a table
 @pytest.mark.parametrize("lkspace,alpha,rc", [(1, 0.05, 10.0), (1, 0.1, 12.0), (1, 0.2, 12.0), (1, 0.24, 10.0),
                                               (2, 0.309, 10.0), (1, 0.35, 10.0), (1, 1.2, 10.0)])
-@pytest.mark.parametrize("energy", [False])
+@pytest.mark.parametrize("energy", [False, True])
 def test_coulomb_of_single_pairs(lkspace, alpha, rc, energy):
     q = 2048.0
     box, pos, r = _pairs(rc, 2.5, 7)
@@ -106,3 +106,27 @@ def test_lj_and_reaction_field_of_single_pairs(energy):
         bound = U * (30 * a + 18 * b + 9 * (c1 + c2)) + 2.0 ** -33
         err = np.abs(f.astype(LD) - ref)
         assert (err <= bound).all(), f"{float((err / bound).max()):.2f} of the bound"
+
+
+@pytest.mark.parametrize("lkspace,alpha", [(1, 0.2), (1, 1.2), (2, 0.309), (0, 0.0)])
+@pytest.mark.parametrize("batch", [False, True])
+def test_forces_do_not_depend_on_energies(lkspace, alpha, batch):
+    """Bit for bit, so that a trajectory does not depend on which steps
+    compute energies."""
+    from md_gpu_gb300 import synth
+    reps = []
+    for k, n in enumerate((998, 1728)):
+        a = synth.to_arrays(synth.nacl_replica(n, seed=3 + k, rc=10.0))
+        a.update(lkspace=lkspace, alfa=alpha, reacf=9e-4 if lkspace == 0 else 0.0)
+        reps.append(a)
+    out = []
+    for every in (0, 1):
+        sim = MDSystem.from_batch(reps) if batch else MDSystem.from_arrays(**reps[0])
+        with sim:
+            sim.set_precision(64)
+            sim.compute_forces(energy=bool(every))
+            f = sim.forces()[:, :3]
+            sim.step(12, every)
+            out.append((f, sim.positions(), sim.velocities()))
+    for p, q in zip(*out):
+        assert np.array_equal(p, q)
