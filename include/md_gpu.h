@@ -132,10 +132,10 @@ md_status md_get_replica_thermo(md_ctx *ctx, md_thermo *out, int nrep);
  * dL/d lj2[a][b] (8x8 per replica, entry a*8+b as used by atoms of type a;
  * the derivative for a symmetric pair parameter is the sum of the (a,b) and
  * (b,a) entries) and dL/d ln s for a common charge scale s, by the discrete
- * adjoint of the integrator, over the positions of every frame when they
- * take at most a quarter of the device's memory (24 bytes per atom and
- * frame), else with (x, v) checkpoints every `checkpoint` steps and
- * recompute.  The context is left at the end of the trajectory.
+ * adjoint of the integrator with (x, v) checkpoints every `checkpoint` steps
+ * and recompute, or over the positions of every frame (24 bytes per atom and
+ * frame) where those take no more memory than the checkpoints and a segment,
+ * or at most 1 GiB.  The context is left at the end of the trajectory.
  * target: nrep*nbins (NULL = 0); loss: nrep; gbar: nrep*nbins (may be NULL);
  * dlj1, dlj2: nrep*64; dlns: nrep. */
 typedef struct {

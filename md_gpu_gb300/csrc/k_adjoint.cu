@@ -643,12 +643,13 @@ extern "C" md_status md_adjoint_run(md_ctx *c, const md_adjoint_cfg *cfg, const 
     const float tab_h = (float)(cfg->rdf_dr / 8.0);
     const int tab_n = (int)(rmax / (double)tab_h) + 3;   /* covers [0, rmax + h] */
     const size_t n3 = 3 * (size_t)n;
-    /* The forward pass keeps every frame's positions when they take at most
-     * a quarter of the device's memory and can be had: the backward pass then
-     * reads them instead of running the trajectory again from checkpoints. */
-    size_t mem_free = 0, mem_total = 0;
-    MD_CUDA_TRY(c, cudaMemGetInfo(&mem_free, &mem_total));
-    bool keep = cfg->gradient && c->adj_keep && sizeof(double) * n3 * (size_t)(K + 1) <= mem_total / 4;
+    /* The forward pass keeps every frame's positions when they take no more
+     * memory than the checkpoints and segment that the caller asked for, or
+     * little (1 GiB, 0.4% of the device's): the backward pass then reads them
+     * instead of running the trajectory again from checkpoints. */
+    const size_t all_frames = sizeof(double) * n3 * (size_t)(K + 1);
+    const size_t segments = sizeof(double) * n3 * (2 * ((size_t)nseg + 1) + (size_t)C + 1);
+    bool keep = cfg->gradient && c->adj_keep && all_frames <= std::max(segments, (size_t)1 << 30);
     auto layout = [&]() {
         B.used = 0;
         B.take(B.ck_x, keep || !cfg->gradient ? 0 : n3 * (nseg + 1));
