@@ -358,7 +358,7 @@ md_status md_set_pme(md_ctx *ctx, int k0, int k1, int k2);
  * of the replicas of a batch after the last md_step (NPT moves them); for a
  * single system its fixed box and pressure 0.  Synchronises the stream. */
 md_status md_get_replica_box(md_ctx *ctx, double *box3, double *pressure_bar, int nrep);
-/* Test hook of the one-kernel list rebuild of a single system (no
+/* Test hook of the one-kernel list rebuild, of a single system or a batch (no
  * counterpart in the reference, whose list build has no grid barriers):
  * its phases are separated by grid barriers whose waits give up after
  * timeout_ms (0: the default, 50 ms) and set a sticky error; with
@@ -368,8 +368,9 @@ md_status md_get_replica_box(md_ctx *ctx, double *box3, double *pressure_bar, in
  * returns without work; the step kernels run on with the list and atom
  * order as the interrupted rebuild left them (every index still in range),
  * and the next synchronising call (md_step, md_update_neighbors, ...)
- * returns MD_ERR_CUDA with the message "a grid barrier of the list rebuild
- * timed out".  The context must then be destroyed (its atom order may be
+ * returns MD_ERR_CUDA with the message "a grid barrier timed out".  The one
+ * launch that runs many steps of a small system has the same limits, and the
+ * dropped block leaves it before its first barrier.  The context must then be destroyed (its atom order may be
  * half permuted); the CUDA context stays usable.  timeout_ms = 0 and drop_block = -1 restore the defaults. */
 md_status md_debug_rebuild_barrier(md_ctx *ctx, double timeout_ms, int drop_block);
 /* Test hook (no counterpart in the reference): gives the list capacity

@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 2) k_run_steps(md_kparams kp, pai
     md_devstate *st = a.st;
     /* the same in every block: written only when a barrier runs out */
     if (*(volatile int *)&st->status != 0) return;
+    if ((int)blockIdx.x == p.bar_drop) return;   /* test hook: the others' waits run out */
     const int t = threadIdx.x;
     const int i0 = blockIdx.x * NA;
     const bool book = blockIdx.x == gridDim.x - 1;   /* the bookkeeping block (no atoms) */
@@ -352,11 +353,11 @@ const void *run_kernel(const md_ctx *c)
 /* Whether md_step runs this system's steps in k_run_steps: a single FP32
  * system without the reciprocal sum whose atoms fit the blocks that are
  * resident at once (two of 256 threads per SM: 9696 atoms at 8 lanes on 152
- * SMs), rebuilt warp per cell.  The test hooks of the one-kernel rebuild and
- * eager launches (md_set_graphs) keep the ordinary path. */
+ * SMs), rebuilt warp per cell.  Eager launches (md_set_graphs) keep the
+ * ordinary path. */
 bool md_can_run_small(md_ctx *c)
 {
-    if (c->batch || c->fp64 || c->pme.on || !c->use_graphs || c->dbg_bar_ns || c->dbg_bar_drop >= 0) return false;
+    if (c->batch || c->fp64 || c->pme.on || !c->use_graphs) return false;
     const void *k = run_kernel(c);
     if (!k || !md_rebuild_coop(c)) return false;
     const int key = c->pair_tpa * 100 + md_pair_depth(c);

@@ -275,7 +275,7 @@ md_status check_overflow_and_sync(md_ctx *c)
                     "boxes (md_get_positions, md_get_replica_box), with a shorter cutoff or skin for the "
                     "latter");
     if (h.status != 0)
-        return fail(c, MD_ERR_CUDA, "a grid barrier of the list rebuild timed out (device state invalid)");
+        return fail(c, MD_ERR_CUDA, "a grid barrier timed out (list rebuild, or the run of a small system's steps; device state invalid)");
     if (h.list_overflow > 0)
         return fail(c, MD_ERR_LIST_OVERFLOW,
                     "neighbour list overflow: " + std::to_string(h.list_overflow) + " > capacity " +
