@@ -392,9 +392,11 @@ md_status md_set_fused_step(md_ctx *ctx, int fused);
 /* How a step graph holds the neighbour-list rebuild (single systems): 0 a
  * conditional node per step whose body is the rebuild; 1 the rebuild inline
  * in every step, launches that return at once when no rebuild is due.  Until
- * this, md_set_fused_step or md_autotune is called, systems too large to run
- * many steps in one launch take 1 (and the fused step where it applies).  Both rebuild at the same
- * steps and give the same trajectory; md_autotune keeps the faster. */
+ * this, md_set_fused_step or md_autotune is called, systems whose steps do not
+ * run many in one launch (at their size, lanes and list builder) take 1 and,
+ * where it applies, the fused step; md_set_fused_step leaves the rebuild as a
+ * new context of the system has it.  Both rebuild at the same steps and give
+ * the same trajectory; md_autotune keeps the faster. */
 md_status md_set_graph_rebuild(md_ctx *ctx, int inline_passes);
 /* Milliseconds of device time of the last md_step call (CUDA events). */
 md_status md_last_step_ms(md_ctx *ctx, float *ms);

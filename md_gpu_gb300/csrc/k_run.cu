@@ -350,14 +350,13 @@ const void *run_kernel(const md_ctx *c)
 
 }  // namespace
 
-/* Whether md_step runs this system's steps in k_run_steps: a single FP32
- * system without the reciprocal sum whose atoms fit the blocks that are
- * resident at once (two of 256 threads per SM: 9696 atoms at 8 lanes on 152
- * SMs), rebuilt warp per cell.  Eager launches (md_set_graphs) keep the
- * ordinary path. */
-bool md_can_run_small(md_ctx *c)
+/* Whether k_run_steps can run this system's steps: a single FP32 system
+ * without the reciprocal sum whose atoms fit the blocks that are resident at
+ * once (two of 256 threads per SM: 9696 atoms at 8 lanes on 152 SMs), rebuilt
+ * warp per cell. */
+bool md_fits_run(md_ctx *c)
 {
-    if (c->batch || c->fp64 || c->pme.on || !c->use_graphs) return false;
+    if (c->batch || c->fp64 || c->pme.on) return false;
     const void *k = run_kernel(c);
     if (!k || !md_rebuild_coop(c)) return false;
     const int key = c->pair_tpa * 100 + md_pair_depth(c);
@@ -372,6 +371,9 @@ bool md_can_run_small(md_ctx *c)
     const int na = RUN_THREADS / c->pair_tpa;
     return (c->n + na - 1) / na + 1 <= c->run_blocks;
 }
+
+/* Whether md_step runs them there (eager launches, md_set_graphs, do not). */
+bool md_can_run_small(md_ctx *c) { return c->use_graphs && md_fits_run(c); }
 
 /* nsteps steps (no energies) in one launch; the positions end in pos4.
  * Returns false when the launch is refused (the caller takes the ordinary

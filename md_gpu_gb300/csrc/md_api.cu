@@ -461,13 +461,17 @@ md_status initial_build(md_ctx *c)
 
 /* The form of the step graphs of a single system that nobody chose
  * (md_autotune, md_set_fused_step, md_set_graph_rebuild): where its steps do
- * not run in k_run_steps, the one-kernel rebuild inline (64000 ions: an idle
- * launch 3 us per step, an idle conditional node 10) and, for leapfrog
- * without bonded terms, pair forces and update as one kernel. */
+ * not run in k_run_steps, the rebuild inline and, for leapfrog without bonded
+ * terms, pair forces and update as one kernel.  us per step behind a
+ * conditional node and separate / inline and fused: 64000 ions 84 / 70 (the
+ * one-kernel rebuild: an idle launch 3, an idle node 10), 982 ions at 4 lanes
+ * 27.3 / 17.3; with another list builder (its chain of passes as programmatic
+ * launches) 982 ions 30.8 / 26.2, 26998 ions 69.4 / 62.6.  Called wherever
+ * what the rule reads changes, with no step graph captured. */
 void default_step_form(md_ctx *c)
 {
     if (c->batch || c->form_chosen) return;
-    const int on = !md_can_run_small(c) && md_rebuild_coop(c) ? 1 : 0;
+    const int on = !md_fits_run(c) ? 1 : 0;
     c->rebuild_inline = on;
     c->fuse_step = on;
 }
@@ -718,8 +722,9 @@ md_status setup_device(md_ctx *c, void *stream, host_stage &h, md_ctx **out)
     md_status s = alloc_list(c, (c->nmaxlist + 31) / 32 * 32);
     if (s == MD_OK) s = initial_build(c);
     if (s == MD_OK) s = refresh_state(c);
-    if (s == MD_OK) default_step_form(c);
     if (s == MD_OK && !c->batch) pick_lanes(c);
+    if (s == MD_OK) default_step_form(c);
+    c->inline_new = c->rebuild_inline;
     if (s != MD_OK) {
         g_last_error = c->last_error;
         md_destroy(c);
@@ -2274,8 +2279,9 @@ md_status md_set_pme(md_ctx *c, int k0, int k1, int k2)
     }
     md_status s = pme_setup(c, K);
     if (s != MD_OK) return s;
-    default_step_form(c);
     if (c->lanes_by_size) pick_lanes(c);
+    default_step_form(c);
+    c->inline_new = c->rebuild_inline;
     return refresh_state(c);   /* the forces (and record) of the current state with the new sum */
 }
 
@@ -2479,6 +2485,7 @@ md_status md_set_precision(md_ctx *c, int bits)
         c->gexec = nullptr;
     }
     default_step_form(c);
+    c->inline_new = c->rebuild_inline;
     /* the forces (and record) of the current state in the new precision */
     return refresh_state(c);
 }
@@ -2526,6 +2533,7 @@ md_status md_set_fused_step(md_ctx *c, int fused)
                     "md_set_fused_step: only leapfrog single systems without bonded terms fuse");
     }
     c->fuse_step = fused ? 1 : 0;
+    if (!c->form_chosen) c->rebuild_inline = c->inline_new;
     c->form_chosen = 1;
     if (c->gexec && c->fuse_step != old) {
         cudaGraphExecDestroy(c->gexec);
@@ -2550,6 +2558,7 @@ md_status md_set_pair_depth(md_ctx *c, int depth)
         cudaGraphExecDestroy(c->gexec);
         c->gexec = nullptr;
     }
+    default_step_form(c);
     return MD_OK;
 }
 
@@ -2568,6 +2577,7 @@ md_status md_set_tuning(md_ctx *c, int pair_tpa, int list_tpa)
         cudaGraphExecDestroy(c->gexec);
         c->gexec = nullptr;
     }
+    default_step_form(c);
     return MD_OK;
 }
 

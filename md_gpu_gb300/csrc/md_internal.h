@@ -253,6 +253,7 @@ struct md_ctx {
     const float4 *gpos4 = nullptr; /* position buffer current when the graph was captured */
     int use_graphs = 1;            /* 0: launch every step's kernels eagerly */
     int form_chosen = 0;           /* 1: the caller or the autotuner chose fuse_step, rebuild_inline */
+    int inline_new = 0;            /* rebuild_inline before any tuning (md_set_fused_step keeps it) */
     int fuse_step = 0;             /* 1: fused pair+leapfrog kernel where applicable */
     int cw_grid[2] = {0, 0};       /* blocks of the persistent list builder (single, batch) */
     int rebuild_coop = 1;          /* single systems: the rebuild as one cooperative kernel */
@@ -400,6 +401,7 @@ bool md_can_fuse(const md_ctx *c);
 void launch_pair_leapfrog(md_ctx *c, const md_kparams &kp, unsigned long long cond, int has_cond);
 
 /* ---- launchers (k_run.cu): many steps of a small system in one launch ---- */
+bool md_fits_run(md_ctx *c);
 bool md_can_run_small(md_ctx *c);
 bool launch_run_steps(md_ctx *c, const md_kparams &kp, int nsteps);
 

@@ -28,3 +28,27 @@ def test_every_depth_matches_separate_kernels(tpa, depth):
             out.append((s.positions(), s.velocities(), s.forces()))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_default_form_follows_the_tuning():
+    """Step graphs that nobody chose a form for: rebuild inline and fused step
+    wherever the steps do not run in one launch, after every setting that
+    changes that; a chosen form stays."""
+    def form(s):
+        i = s.info()
+        return bool(i["rebuild_inline"]), bool(i["fused_step"])
+
+    for natom, tunings in ((982, (((4, 0), True), ((8, 0), False), ((8, 8), True), ((32, 0), False))),
+                           (9602, (((16, 0), True), ((8, 0), False), ((8, 4), True))),
+                           (13822, (((8, 8), True), ((8, 0), True), ((16, 0), True)))):
+        with MDSystem.from_arrays(**_nacl(natom)) as s:
+            assert form(s) == ((natom > 9696),) * 2
+            for (tpa, ltpa), on in tunings:
+                s.set_tuning(tpa, ltpa)
+                assert form(s) == (on, on), (natom, tpa, ltpa)
+                s.step(6)
+            s.set_fused_step(False)
+            s.set_graph_rebuild(False)
+            s.set_tuning(4, 0)
+            assert form(s) == (False, False)
+            s.step(6)
