@@ -300,7 +300,11 @@ md_status md_set_pair_depth(md_ctx *ctx, int depth);
  * times the step graphs by running steps: fused or separate pair and
  * integrator kernels (leapfrog systems without bonded terms), and for single
  * systems the rebuild inline or behind a conditional node
- * (md_set_graph_rebuild), each for the three fastest pair settings.  The
+ * (md_set_graph_rebuild), each for the three fastest pair settings.  A system
+ * whose steps can run many in one launch is timed so, at 8 and 16 lanes, and
+ * against the fastest other setting's graphs; it keeps the warp-per-cell
+ * builder that the launch needs if that wins (the 32 lanes that the smallest
+ * systems are created with are not among the settings).  The
  * system advances 128 steps per combination tried (up to 12; batches have
  * one and do not advance). */
 md_status md_autotune(md_ctx *ctx, int *pair_tpa, int *list_tpa);

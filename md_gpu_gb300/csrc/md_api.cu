@@ -2300,18 +2300,23 @@ md_status md_autotune(md_ctx *c, int *pair_tpa, int *list_tpa)
     if (!c) return MD_ERR_ARG;
     c->form_chosen = 1;
     c->lanes_by_size = 0;
+    c->list_tpa = 0;   /* chosen last */
     const int lt[] = {0, 4, 8, 16};
     float best = 1e30f;
-    int bp = c->pair_tpa, bl = c->list_tpa, bf = 0;
+    int bl = 0, bf = 0;
     c->fuse_step = 0;
     /* best of three timings of 20 launches per candidate (lanes per atom,
      * entries per lane and batch): robust to a slow first launch and to other
      * work on the device. */
     const int combos[][2] = {{2, 0}, {4, 0}, {4, 4}, {8, 0}, {8, 2}, {16, 0}, {16, 1}};
-    std::vector<std::pair<float, int>> ranked;   /* (ms, combo) */
-    for (int q = 0; q < (int)(sizeof(combos) / sizeof(combos[0])); q++) {
+    const int ncombo = (int)(sizeof(combos) / sizeof(combos[0]));
+    auto set = [&](int q) {
         c->pair_tpa = combos[q][0];
         c->pair_depth = combos[q][1];
+    };
+    std::vector<std::pair<float, int>> ranked;   /* (ms, combo) */
+    for (int q = 0; q < ncombo; q++) {
+        set(q);
         float ms = 0.0f, m2 = 1e30f;
         md_status s = md_time_pair(c, 5, &ms);
         for (int rep = 0; rep < 3 && s == MD_OK; rep++) {
@@ -2323,55 +2328,73 @@ md_status md_autotune(md_ctx *c, int *pair_tpa, int *list_tpa)
     }
     std::sort(ranked.begin(), ranked.end());
     int bq = ranked[0].second;
-    c->pair_tpa = combos[bq][0];
-    c->pair_depth = combos[bq][1];
+    set(bq);
+    /* What step times are compared for.  Where some lanes let many steps run in
+     * one launch (k_run_steps), which takes no step graph and reads neither
+     * its form nor, between two and four entries, the depth: each such lane
+     * count once, and the fastest of the other pair settings.  Else the three
+     * fastest pair settings (the fused kernel's own ranking may differ). */
+    std::vector<int> cand, other;
+    int seen = 0;
+    for (const auto &r : ranked) {
+        set(r.second);
+        const int kind = 1 << (2 * (c->pair_tpa / 16) + md_pair_depth(c) % 2);   /* lanes 8 or 16; depth odd */
+        if (!md_can_run_small(c)) other.push_back(r.second);
+        else if (!(seen & kind)) {
+            seen |= kind;
+            cand.push_back(r.second);
+        }
+    }
+    const bool runs = !cand.empty();
+    for (size_t k = 0; k < other.size() && k < (runs ? 1 : 3); k++) cand.push_back(other[k]);
     /* the step graph: separate or (leapfrog without bonded terms) fused pair
      * and integrator kernels, the rebuild behind a conditional node or inline
-     * (single systems), for the three fastest pair settings (the fused
-     * kernel's own ranking may differ); each combination timed as it runs,
-     * 96 steps after 32 of warm-up, less the list builds that fell in the
-     * window at the measured cost of one (the system advances 128 steps per
-     * combination) */
+     * (single systems); each combination timed as it runs, 96 steps after 32
+     * of warm-up, less the list builds that fell in the window at the measured
+     * cost of one (the system advances 128 steps per combination) */
     int bi = 0;
     c->fuse_step = 1;
     const int nf = md_can_fuse(c) ? 2 : 1, ni = c->batch ? 1 : 2;
+    bool brun = false;
     if (nf * ni > 1) {   /* a batch has one choice: it keeps its state */
         float t_rb = 0.0f;
+        set(ranked[0].second);
         md_status s = md_time_rebuild(c, 3, &t_rb);
         if (s != MD_OK) return s;
         float tbest = 1e30f;
-        for (int cand = 0; cand < std::min(3, (int)ranked.size()); cand++)
-        for (int fz = 0; fz < nf; fz++)
-            for (int inl = 0; inl < ni; inl++) {
-                const int q = ranked[cand].second;
-                c->pair_tpa = combos[q][0];
-                c->pair_depth = combos[q][1];
-                c->fuse_step = fz;
-                c->rebuild_inline = inl;
-                if (c->gexec) {
-                    cudaGraphExecDestroy(c->gexec);
-                    c->gexec = nullptr;
+        for (int q : cand) {
+            set(q);
+            const bool run = md_can_run_small(c);
+            /* (steps of the run's context that do need a graph take the form
+             * that is faster wherever it was measured) */
+            for (int fz = run ? nf - 1 : 0; fz < nf; fz++)
+                for (int inl = run ? ni - 1 : 0; inl < ni; inl++) {
+                    c->fuse_step = fz;
+                    c->rebuild_inline = inl;
+                    if (c->gexec) {
+                        cudaGraphExecDestroy(c->gexec);
+                        c->gexec = nullptr;
+                    }
+                    s = md_step(c, 32, 0);
+                    int b0 = 0, b1 = 0;
+                    float ms = 0.0f;
+                    if (s == MD_OK) s = read_builds(c, &b0);
+                    if (s == MD_OK) s = md_step(c, 96, 0);
+                    if (s == MD_OK) s = md_last_step_ms(c, &ms);
+                    if (s == MD_OK) s = read_builds(c, &b1);
+                    if (s != MD_OK) return s;
+                    const float t = ms - (float)(b1 - b0) * t_rb;
+                    if (t < tbest) { tbest = t; bf = fz; bi = inl; bq = q; brun = run; }
                 }
-                s = md_step(c, 32, 0);
-                int b0 = 0, b1 = 0;
-                float ms = 0.0f;
-                if (s == MD_OK) s = read_builds(c, &b0);
-                if (s == MD_OK) s = md_step(c, 96, 0);
-                if (s == MD_OK) s = md_last_step_ms(c, &ms);
-                if (s == MD_OK) s = read_builds(c, &b1);
-                if (s != MD_OK) return s;
-                const float t = ms - (float)(b1 - b0) * t_rb;
-                if (t < tbest) { tbest = t; bf = fz; bi = inl; bq = q; }
-            }
+        }
     }
-    bp = combos[bq][0];
-    c->pair_tpa = bp;
-    c->pair_depth = combos[bq][1];
+    set(bq);
     c->fuse_step = bf;
     c->rebuild_inline = bi;
     best = 1e30f;
     for (int t : lt) {
         if (c->batch && t != 0) continue;   /* batches build one warp per cell */
+        if (brun && t != 0) continue;       /* so does the run of steps in one launch */
         c->list_tpa = t;
         float ms = 0.0f, m2 = 1e30f;
         md_status s = md_time_rebuild(c, 2, &ms);
@@ -2387,7 +2410,7 @@ md_status md_autotune(md_ctx *c, int *pair_tpa, int *list_tpa)
         cudaGraphExecDestroy(c->gexec);
         c->gexec = nullptr;
     }
-    if (pair_tpa) *pair_tpa = bp;
+    if (pair_tpa) *pair_tpa = c->pair_tpa;
     if (list_tpa) *list_tpa = bl;
     return MD_OK;
 }

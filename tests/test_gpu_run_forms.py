@@ -52,3 +52,29 @@ def test_default_form_follows_the_tuning():
             s.set_tuning(4, 0)
             assert form(s) == (False, False)
             s.step(6)
+
+
+@pytest.mark.parametrize("natom", [510, 982, 4080, 9602])
+def test_autotuned_small_system_runs_in_one_launch(natom):
+    """With a block dropped (test hook) and no rebuild due, steps time out in
+    the one launch only: the separate kernels have no wait then."""
+    from md_gpu_gb300.system import MDError, library
+    with MDSystem.from_arrays(**_nacl(natom)) as s:
+        s.step(16)
+        s.autotune()
+        i = s.info()
+        assert i["list_tpa"] == 0 and i["pair_tpa"] >= 8
+        s.update_neighbors(force=True)
+        assert library().md_debug_rebuild_barrier(s._ctx, 2.0, 0) == 0
+        with pytest.raises(MDError):
+            s.step(4)
+
+
+def test_control_of_the_above():
+    from md_gpu_gb300.system import library
+    with MDSystem.from_arrays(**_nacl(982)) as s:
+        s.step(16)
+        s.set_tuning(4, 0)
+        s.update_neighbors(force=True)
+        assert library().md_debug_rebuild_barrier(s._ctx, 2.0, 0) == 0
+        s.step(4)
