@@ -432,9 +432,11 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_build_cells(
 __global__ void __launch_bounds__(CW_WARPS * 32, 2) k_rebuild_coop(md_kparams kp, md_devstate *st, int always,
                                                                 rb_ptrs p)
 {
-    /* the same in every block: nothing writes either before the end; a
-     * status left by an earlier launch (a barrier that timed out, whose
-     * arrival count is then stale) stops every later rebuild */
+    /* the same in every block: the request is cleared after the first
+     * barrier, which every block reaches only after reading it, and the status
+     * written only when a wait runs out; one left by an earlier launch (a
+     * barrier that timed out, whose arrival count is then stale) stops every
+     * later rebuild */
     if (!always && !st->update) return;
     if (*(volatile int *)&st->status != 0) return;
     grid_bar bar = {st, gridDim.x, p.bar_ns, 0ull};

@@ -1590,10 +1590,12 @@ static md_status sync_reps(md_ctx *c)
 
 /* Steps of a small system from here on that k_run_steps takes in one
  * launch: up to the next step with energies (which runs as separate
- * kernels), at most 1024 (a few ms), at least 4. */
+ * kernels), at least 4, at most 256: 2 to 7 ms (6 to 27 us per step), within
+ * which kernels of other contexts find only the SM slots it leaves.  A launch
+ * more per 256 steps is about 5 us. */
 static int run_small_steps(md_ctx *c, int left, int energy_every)
 {
-    int k = std::min(left, 1024);
+    int k = std::min(left, 256);
     if (energy_every > 0) {
         const long long past = c->host_step % energy_every;
         if (past == 0) return 0;

@@ -78,3 +78,43 @@ def test_control_of_the_above():
         s.update_neighbors(force=True)
         assert library().md_debug_rebuild_barrier(s._ctx, 2.0, 0) == 0
         s.step(4)
+
+
+@pytest.mark.parametrize("sizes", [(982, 982, 982), (9602, 9602), (982, 13822)])
+def test_contexts_stepped_at_once(sizes):
+    """Contexts of several threads at work together, each launch needing its
+    blocks resident (9602 ions: nearly the whole device each): the same bits
+    as one after the other, runs of more than one launch among them."""
+    def make(k, n):
+        return MDSystem.from_arrays(**_nacl(n, seed=4 + k))
+
+    def go(s):
+        for n in (300, 7, 64):
+            s.step(n)
+
+    alone = []
+    for k, n in enumerate(sizes):
+        with make(k, n) as s:
+            go(s)
+            alone.append(s.positions())
+    sims = [make(k, n) for k, n in enumerate(sizes)]
+    errors = []
+
+    def work(s):
+        try:
+            go(s)
+        except Exception as e:   # raised in the test's own thread below
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in sims]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    try:
+        assert not errors, errors
+        for s, p in zip(sims, alone):
+            assert np.array_equal(s.positions(), p)
+    finally:
+        for s in sims:
+            s.close()
