@@ -228,13 +228,13 @@ struct wrap2 {
  * vary per entry run on v2; those with a per-atom or per-system constant run
  * as scalar IEEE operations with the constant (no register pair to hold it).
  * The same formulas as pair_term, with every rounding step fixed, and the
- * same forces with and without ENERGY (pair_sum takes it for the Wolf form
- * then). */
+ * same forces with and without ENERGY (the Wolf form only: pair_sum). */
 template <int KIND, bool ENERGY, bool WRAP, bool PACKED, class G>
 __device__ __forceinline__ void pair_term2(const G &g, const wrap2<PACKED> &W, v2<PACKED> PX, v2<PACKED> PY,
                                            v2<PACKED> PZ, float qi, float4 p0, float4 p1, float2 l0,
                                            float2 l1, pair_acc2<PACKED> &a)
 {
+    static_assert(KIND == 1 || !ENERGY, "energies of the reaction field go through pair_term");
     typedef v2<PACKED> V;
     V dx = PX - V::make(p0.x, p1.x), dy = PY - V::make(p0.y, p1.y), dz = PZ - V::make(p0.z, p1.z);
     if (WRAP) {
@@ -273,10 +273,6 @@ __device__ __forceinline__ void pair_term2(const G &g, const wrap2<PACKED> &W, v
         float a0, a1;
         ri.get(a0, a1);
         ff = qq * V::make(__fmaf_rn(-g.reacf(), s0, a0), __fmaf_rn(-g.reacf(), s1, a1));
-        if (ENERGY) {
-            u0 = qq0 * (a0 + 0.5f * g.reacf() * s0 - g.ucc());
-            u1 = qq1 * (a1 + 0.5f * g.reacf() * s1 - g.ucc());
-        }
     }
     const V ri6 = ri2 * ri2 * ri2;
     float m0, m1;
@@ -367,7 +363,7 @@ __device__ __forceinline__ void pair_loop(const G &g, float4 pi, float qi, int n
         for (int b = 0; b < B; b++) p[b] = ld_list<NC>(pos4 + (e[b] & MD_INDEX_MASK));
     };
     auto eval = [&](const float4 (&p)[B], const unsigned (&e)[B]) {
-        if (PACK && B % 2 == 0) {
+        if constexpr (PACK && B % 2 == 0) {
 #pragma unroll
             for (int b = 0; b < B; b += 2)
                 pair_term2<KIND, ENERGY, WRAP, true>(g, W, PX, PY, PZ, qi, p[b], p[b + 1], ljrow[e[b] >> MD_TYPE_SHIFT],

@@ -741,7 +741,7 @@ struct grid_bar {
 /* The arrays the rebuild passes touch. */
 struct rb_ptrs {
     const int *cell_rank, *cell_lin;
-    int *key, *cell_count, *cell_start, *cell_fill, *src;
+    int *key, *cell_count, *cell_start, *src;
     double *x, *v, *mass, *kick, *tmp_d;
     float4 *pos4, *tmp4, *pos_old;
     int *perm, *iperm, *type, *tmp_i;
@@ -784,7 +784,6 @@ inline rb_ptrs make_rb_ptrs(const md_ctx *c, int blocks)
     p.key = c->key;
     p.cell_count = c->cell_count;
     p.cell_start = c->cell_start;
-    p.cell_fill = c->cell_fill;
     p.src = c->src;
     p.x = c->x;
     p.v = c->v;
