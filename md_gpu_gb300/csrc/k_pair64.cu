@@ -339,21 +339,22 @@ __global__ void k_bonded64(int n, int pitch, const double *__restrict__ boxd,
  * e^{-a^2 r^2}, t = 1 / (1 + p a r): on each the Chebyshev interpolant of
  * degree MD_P64_DEG, written in powers of r - centre and computed in long
  * double, so that its coefficients are as good as FP64 holds them.  Takes the
- * fewest pieces whose largest deviation at 16 points a piece is at most 1e-16,
- * an ulp of G just below 1 (G as written, evaluated in FP64, is off by 4e-16
- * to 8e-16; at 4e-15, the line before, the pieces were the larger error); none:
- * m.ni = 0. */
+ * fewest pieces whose deviation at four extrema of the next Chebyshev
+ * polynomial, the shape of the error, is at most 1e-16, an ulp of G just below
+ * 1 (G as written, evaluated in FP64, is off by 4e-16 to 8e-16; at 4e-15, the
+ * line before, the pieces were the larger error); none: m.ni = 0. */
 static void fit_coulomb(md_p64 &m)
 {
     typedef long double real;
-    constexpr int N = MD_P64_DEG + 1, CHK = 16;
+    constexpr int N = MD_P64_DEG + 1, CHK = 4;
     auto G = [&](real r) {
         const real xa = m.alpha * r, t = 1.0L / (1.0L + m.pex * xa);
         const real p = ((((m.a[4] * t + m.a[3]) * t + m.a[2]) * t + m.a[1]) * t + m.a[0]);
         const real ex = expl(-xa * xa);
         return p * t * ex + m.spi * r * ex;
     };
-    const real pi = acosl(-1.0L);
+    const real pi = acosl(-1.0L), chk[CHK] = {-1.0L, cosl(5.0L * pi / 8.0L), cosl(3.0L * pi / 8.0L), 1.0L};
+    static_assert(MD_P64_DEG == 7, "chk are extrema of T_8");
     /* T_j at the nodes, weighted, and (monomial) T_j's coefficients */
     real node[N], tj[N][N], mono[N][N] = {};
     for (int k = 0; k < N; k++) {
@@ -376,7 +377,7 @@ static void fit_coulomb(md_p64 &m)
                 for (int k = 0; k <= j; k++) c[k] += a * mono[j][k];
             }
             for (int k = 0; k < CHK && ok; k++) {
-                const real y = -1.0L + (2 * k + 1) / (real)CHK;
+                const real y = chk[k];
                 real g = 0.0L;
                 for (int d = N - 1; d >= 0; d--) g = g * y + c[d];
                 ok = fabsl(g - G(cen + h * y)) <= 1e-16L;
