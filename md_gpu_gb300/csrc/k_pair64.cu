@@ -61,7 +61,7 @@ __device__ __forceinline__ double rsqrt64(double s, float &seed)
  * instruction in 20 cycles, so its operations are what counts: the force's
  * Coulomb term comes from a piecewise polynomial (tab, 8 FP64 operations;
  * exp and the divide of the A&S form, which the energy takes, over 40).  4082 ions,
- * per launch: 230 us as written, 102 us so.  Its argument r - centre is one
+ * per launch: 230 us as written, 102 us so (77% of the FP64 pipe).  Its argument r - centre is one
  * fma of r^2 and 1/r: r itself is never rounded.  Against quad precision, at
  * distances from 1.5 A to rc (a rc 0.5 to 3.2): the largest error of G 1.2e-16
  * to 2.3e-16 (rms 4e-17), the form as written in FP64 4.1e-16 to 7.7e-16 (rms

@@ -117,8 +117,8 @@ __global__ void k_pme_prep(pme_par pp, const double *__restrict__ x, const float
  * queue each atom whose spline reaches the brick (spline origin relative to
  * the brick, its 12 weights, charge).  A queue that might not hold the next
  * round, and the last one, is deposited: each lane adds one (atom, x, y) row
- * of four z points per pass.  Bound by latency, so few rounds and few
- * barriers count, and few instructions: 64000 ions, 112^3, per launch 32 us
+ * of four z points per pass.  Bound by issue slots (80% busy) and the rounds'
+ * barriers, so few instructions count, and few rounds: 64000 ions, 112^3, per launch 32 us
  * with a prefix sum by one warp, a search per candidate, the 64 cells of the
  * widest brick, a deposit per 256 candidates and 64-bit conversions; 25 us
  * so. */
@@ -510,8 +510,8 @@ void pme_free(md_ctx *c)
 }
 
 /* The convolution runs on a stream of its own beside the pair and bonded
- * kernels, which it shares no data with: it is bound by latency (bricks,
- * small transforms), they by issue slots.  64000 ions, 112^3 grid, per step:
+ * kernels, which it shares no data with: most of it (small transforms, the
+ * solve) is bound by latency, they by issue slots.  64000 ions, 112^3 grid, per step:
  * 161 us in line, 148 beside. */
 void launch_pme_start(md_ctx *c, const md_kparams &kp)
 {

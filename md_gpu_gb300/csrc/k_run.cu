@@ -25,12 +25,13 @@
  * operation, so a run is bit for bit the same.
  *
  * What bounds it is latency: the chain list entry -> position -> force ->
- * update -> barrier of one step, and the rebuilds.  Whole md_step calls of
+ * update -> barrier of one step, and the rebuilds (issue slots 18% busy at 982
+ * ions and 32 lanes, 30% at 4080 and 16).  Whole md_step calls of
  * 100 steps against the step graphs: 500 LJ atoms 2.48 -> 0.83 ms, 4000 LJ
- * atoms 2.71 -> 1.01 ms, 982 ions 3.30 -> 1.01 ms; 20 steps of 5184 water
+ * atoms 2.71 -> 1.00 ms, 982 ions 3.30 -> 1.01 ms; 20 steps of 5184 water
  * atoms 1.58 -> 0.74 ms.  Above the resident
- * blocks the step graphs are the only form (8000 ions: 16.2 us per step here,
- * 28.4 with 16 lanes per atom, where they do not fit).  Copying the block's
+ * blocks the step graphs are the only form (7998 ions: 16.4 us per step here,
+ * 20.4 with 16 lanes per atom, where they do not fit).  Copying the block's
  * list rows to shared memory at each rebuild was no faster (12.8 against
  * 12.0 us per step for 982 ions at 8 lanes), nor was copying all positions
  * there each step (2048 LJ atoms: 8.5 against 7.6).

@@ -561,11 +561,11 @@ struct host_stage {
  * run of steps in one launch (k_run.cu: blocks of 256 / lanes atoms and one
  * more) has one block per SM at 32 lanes or two at 16, else 8.  A small
  * system's step is a chain of latencies, and more lanes shorten the part of
- * it that walks a row.  us per step at 8 / 16 / 32 lanes: 982 ions 12.0 / 9.5
- * / 9.0, 1536 water atoms 18.5 / 14.4 / 15.4, 4080 ions 12.9 / 11.6 / 26 (too
- * many blocks), 8000 ions 16.2 / 28.4 / - .  Rows expected to hold fewer than
+ * it that walks a row.  us per step at 8 / 16 / 32 lanes: 982 ions 12.2 / 9.8
+ * / 8.9, 1536 water atoms 19.1 / 15.0 / 15.4, 4080 ions 13.0 / 11.8 / 16.7
+ * (too many blocks: step graphs), 7998 ions 16.4 / 20.4 / 23.7.  Rows expected to hold fewer than
  * 128 entries keep 8 lanes: an LJ liquid's (80 entries at rc 2.5 sigma) gain
- * less (500 atoms 7.1 / 6.4 / 6.3, 4000 atoms 7.9 / 7.8 / -), and its
+ * less (500 atoms 7.3 / 6.6 / 6.3, 4000 atoms 8.0 / 7.5 / 14.2), and its
  * trajectories amplify a change in the order of the FP32 sums the most (to
  * 1e-5 of the velocities in 100 steps).  With the reciprocal sum, whose kernels
  * run beside the pair kernel, 16 at most: 1000 ions 45.5 / 45.0 / 49.0, 2744

@@ -1,8 +1,7 @@
 /*
  * md_rebuild.cuh -- the neighbour-list rebuild of a single system as phases
- * of one kernel: binning, one-block scan, scatter, in-cell order, permute,
- * copy-back, remap and the warp-per-cell list build, separated by a grid
- * barrier that the kernel brings.  k_rebuild_coop (k_cells.cu) is these
+ * of one kernel: binning, scan, scatter, permute, then copy-back, remap and
+ * the list build, separated by a grid barrier that the kernel brings.  k_rebuild_coop (k_cells.cu) is these
  * phases alone; k_run_steps (k_run.cu) runs them between its steps.
  */
 #ifndef MD_REBUILD_CUH
@@ -242,8 +241,10 @@ __device__ __forceinline__ void remap_one(const md_kparams &kp, int s, const int
  * land in the same order as in k_build_list (stencil cells in traversal order, ascending
  * j) whatever the parts, so all builders produce identical lists.
  *
- * It is bound by issue slots.  Per build against one warp per cell with a
- * 32-wide queue: 64000 ions 149 -> 122 us (102 M -> 66 M warp instructions;
+ * At 16 warps per SM it is bound by their chains of ballots, shuffles and
+ * loads (issue slots 46% busy, stalls per issue long scoreboard 1.9, wait 1.8,
+ * barrier 1.3), so fewer instructions per candidate count.  Per build against
+ * one warp per cell with a 32-wide queue: 64000 ions 149 -> 122 us (102 M -> 66 M warp instructions;
  * the whole rebuild kernel), 982 ions (64 cells, split in parts) 106 -> 39
  * us, 5184 water atoms (exclusions) 476 -> 91 us, 128 replicas of 512 to
  * 8000 ions 834 -> 762 us.  Two blocks of 8 warps per SM at 128 registers:
